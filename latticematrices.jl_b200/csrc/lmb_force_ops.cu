@@ -1,6 +1,7 @@
 // lmb_force_ops.cu -- HISQ smearing chain (Fat7 / Lepage, U(3) projection,
 // Naik), the HISQ and Wilson-clover link pullbacks and fermion forces.
 #include "lmb_clover_force.cuh"
+#include "lmb_fat7.cuh"
 #include "lmb_hisq_force.cuh"
 #include "lmb_op_staggered.cuh"
 #include "lmb_op_wilson.cuh"
@@ -9,34 +10,106 @@ using namespace lmb;
 
 namespace lmb {
 
+// extent of a block of sites along an axis of n sites: the one of `most`, most
+// - 1, .. (most + 1) / 2 that leaves the fewest idle lanes in the last block
+int block_extent(int n, int most) {
+  if (n <= most) return n;
+  int best = most;
+  for (int t = most - 1; 2 * t > most; t--)
+    if ((n + t - 1) / t * t < (n + best - 1) / best * best) best = t;
+  return best;
+}
+// A block of up to kFat7Threads sites, long first in x (whole lines of eight
+// sites), then along the axes of `order` in turn: those along which the
+// kernel's matrices are read again by the neighbour.  With four sites along
+// both axes of a transport, half of its six gathered matrices hit L1.
+SiteTile fat7_tile(const Geom &g, const int *order, int norder) {
+  SiteTile t{{1, 1, 1, 1}, {0, 0, 0, 0}};
+  t.t[0] = block_extent(g.L[0], 8);
+  int left = kFat7Threads / t.t[0];
+  for (int pass = 0; pass < 2; pass++)
+    for (int i = 0; i < norder; i++) {
+      const int d = order[i];
+      if (d == 0) continue;
+      const int now = t.t[d];
+      const int most = std::min(pass ? 8 : 4, left * now);
+      if (most <= now) continue;
+      t.t[d] = std::max(now, block_extent(g.L[d], most));
+      left = left * now / t.t[d];
+    }
+  for (int d = 0; d < 4; d++) t.n[d] = (g.L[d] + t.t[d] - 1) / t.t[d];
+  return t;
+}
+unsigned blocks_of(const SiteTile &t) { return (unsigned)t.n[0] * t.n[1] * t.n[2] * t.n[3]; }
+
+struct Fat7Launch {
+  int nmu;  // directions per launch
+  int64_t per_mu;
+};
+// Directions per launch.  One direction's three axes give V / 128 x 3 blocks;
+// below 64 Ki sites that is less than about four waves of the 148 SMs, and
+// the four directions share a launch (their workspaces then hold at most
+// 700 MB); larger lattices keep one direction's workspace.
+Fat7Launch fat7_launch(const Geom &g, int fields) {
+  return Fat7Launch{g.V <= (1 << 16) ? 4 : 1, (int64_t)fields * 9 * g.V};
+}
+
+// block shapes of a stage for the directions mu0 .. mu0 + nmu - 1, and the
+// largest number of blocks
+enum Fat7Stage { F7_THREE, F7_FIVE, F7_SUM, F7_GRAD };
+unsigned fat7_tiles(const Geom &g, Fat7Stage stage, int mu0, int nmu, Fat7Tiles &tl) {
+  unsigned most = 0;
+  for (int i = 0; i < nmu; i++)
+    for (int slot = 0; slot < 3; slot++) {
+      const int mu = mu0 + i;
+      int ax[3], k = 0;
+      for (int d = 0; d < 4; d++)
+        if (d != mu) ax[k++] = d;
+      const int a = slot == 0 ? 1 : 0, c = slot == 2 ? 1 : 2;
+      const int three[4] = {ax[slot], mu, ax[a], ax[c]}, five[4] = {ax[a], ax[c], mu, ax[slot]};
+      const int sum[4] = {mu, ax[0], ax[1], ax[2]}, grad[4] = {mu, ax[2], ax[1], ax[0]};
+      const int *order = stage == F7_THREE ? three : stage == F7_FIVE ? five : stage == F7_SUM ? sum : grad;
+      tl.t[i][slot] = fat7_tile(g, order, 4);
+      most = std::max(most, blocks_of(tl.t[i][slot]));
+    }
+  return most;
+}
+
+template <int NF, bool LEPAGE>
+void fat7_staples(lmb_ctx *ctx, const Fat7Launch &l, const double2 *U, const Fat7Field &f0, const Fat7Field &f1,
+                  int mu0, const double *coef, cudaStream_t st) {
+  Fat7Tiles tl;
+  unsigned n = fat7_tiles(ctx->g, F7_THREE, mu0, l.nmu, tl);
+  fat7_three_kernel<NF, LEPAGE><<<dim3(3 * n, l.nmu), kFat7Threads, 0, st>>>(ctx->g, tl, U, f0, f1, mu0, l.per_mu);
+  n = fat7_tiles(ctx->g, F7_FIVE, mu0, l.nmu, tl);
+  fat7_five_kernel<NF, LEPAGE><<<dim3(3 * n, l.nmu), kFat7Threads, 0, st>>>(ctx->g, tl, U, f0, f1, mu0, l.per_mu,
+                                                                            coef[2], coef[3], coef[4]);
+}
+
+template <bool ACCUMULATE>
+void fat7_sum(lmb_ctx *ctx, const Fat7Launch &l, const double2 *U, double2 *out, const Fat7Field &f, int mu0,
+              double c1, cudaStream_t st) {
+  Fat7Tiles tl;
+  const unsigned n = fat7_tiles(ctx->g, F7_SUM, mu0, l.nmu, tl);
+  fat7_sum_kernel<ACCUMULATE><<<dim3(n, l.nmu), kFat7Threads, 0, st>>>(ctx->g, tl, U, out, f, mu0, l.per_mu, c1);
+}
+
 // V = Fat7(U) with coefficients (c1, c3, c5, c7, cLepage)
 int fat7_planes(lmb_ctx *ctx, const double2 *U, double2 *V, const double *coef, cudaStream_t st) {
-  const int64_t n = ctx->g.V;
-  double2 *work = (double2 *)workspace(ctx, "smear_staples", sizeof(double2) * 54 * n);
+  const int64_t F3 = 27 * ctx->g.V;  // the three axes' fields
+  const bool lepage = coef[4] != 0.0;
+  const int fields = lepage ? 9 : 6;
+  const Fat7Launch l = fat7_launch(ctx->g, fields);
+  double2 *work = (double2 *)workspace(ctx, "fat7", sizeof(double2) * l.nmu * l.per_mu);
   if (!work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing staples)");
-  double2 *S3[3] = {work, work + 9 * n, work + 18 * n};
-  double2 *S5[3] = {work + 27 * n, work + 36 * n, work + 45 * n};
-  const unsigned grid = grid_for(n, kSmearThreads);
-  for (int mu = 0; mu < 4; mu++) {
-    int axes[3], k = 0;
-    for (int d = 0; d < 4; d++)
-      if (d != mu) axes[k++] = d;
-    const double2 *Umu = U + (size_t)mu * 9 * n;
-    double2 *Vmu = V + (size_t)mu * 9 * n;
-    for (int slot = 0; slot < 3; slot++)
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(S3[slot], Umu, U, ctx->g, mu, axes[slot], 3, 0, 1.0);
-    for (int slot = 0; slot < 3; slot++) {
-      const int bs = slot == 0 ? 1 : 0, cs = slot == 2 ? 1 : 2;
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(S5[slot], S3[cs], U, ctx->g, mu, axes[bs], 3, 0, 1.0);
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(S5[slot], S3[bs], U, ctx->g, mu, axes[cs], 3, 1, 1.0);
-    }
-    fat7_combine_kernel<<<grid_for(9 * n, 256), 256, 0, st>>>(Vmu, Umu, S3[0], S3[1], S3[2], S5[0], S5[1], S5[2],
-                                                               n, coef[0], coef[1], coef[2]);
-    for (int slot = 0; slot < 3; slot++)
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(Vmu, S5[slot], U, ctx->g, mu, axes[slot], 3, 1,
-                                                              coef[3]);
+  const Fat7Field f{U, work, work + F3, lepage ? work + 2 * F3 : work + F3, coef[1]};
+  for (int mu = 0; mu < 4; mu += l.nmu) {
+    if (lepage)
+      fat7_staples<1, true>(ctx, l, U, f, f, mu, coef, st);
+    else
+      fat7_staples<1, false>(ctx, l, U, f, f, mu, coef, st);
+    fat7_sum<false>(ctx, l, U, V, f, mu, coef[0], st);
   }
-  if (coef[4] != 0.0) lepage_kernel<<<grid_for(4 * n, kSmearThreads), kSmearThreads, 0, st>>>(V, U, ctx->g, coef[4]);
   LMB_CHECK_LAUNCH(ctx);
   return LMB_OK;
 }
@@ -53,14 +126,18 @@ int naik_planes(lmb_ctx *ctx, const double2 *W, double2 *L, cudaStream_t st) {
   return LMB_OK;
 }
 
-// install 36-plane links as a link set of the context (derived, not uploaded)
-int install_links(lmb_ctx *ctx, int which, const double2 *planes, cudaStream_t st) {
+// storage of a derived (not uploaded) link set, to be written in place and
+// then installed
+double2 *derived_planes(lmb_ctx *ctx, int which) {
   LinkSet &ls = ctx->links[which];
-  const int64_t V = ctx->g.V;
-  if (!ls.d) LMB_CUDA(ctx, cudaMalloc(&ls.d, sizeof(double2) * 36 * V));
-  LMB_CUDA(ctx, cudaMemcpyAsync(ls.d, planes, sizeof(double2) * 36 * V, cudaMemcpyDeviceToDevice, st));
+  ls.valid = false;
+  if (!ls.d && cudaMalloc(&ls.d, sizeof(double2) * 36 * ctx->g.V) != cudaSuccess) ls.d = nullptr;
+  return ls.d;
+}
+int install_links(lmb_ctx *ctx, int which, cudaStream_t st) {
+  LinkSet &ls = ctx->links[which];
   int rc;
-  ls.scale = device_absmax(ctx, ls.d, 36 * V, st, &rc);
+  ls.scale = device_absmax(ctx, ls.d, 36 * ctx->g.V, st, &rc);
   if (rc) return rc;
   ls.su3_dev = 1.0;  // smeared links are not SU(3): never reconstruct
   for (int mu = 0; mu < 4; mu++) {
@@ -72,78 +149,27 @@ int install_links(lmb_ctx *ctx, int which, const double2 *planes, cudaStream_t s
   return LMB_OK;
 }
 
-// ---------------------------------------------------------------------------
-// HISQ force: reverse pass of the factorised Fat7 with staple recomputation
-// ---------------------------------------------------------------------------
+// dU += d/dU Re<dV, Fat7(U)>: the staples of U and of dV, the Fat7 map of dV
+// onto its own direction, and the transports' links
 int fat7_pullback_planes(lmb_ctx *ctx, const double2 *U, const double2 *dV, double2 *dU, const double *coef,
                          cudaStream_t st) {
-  const int64_t n = ctx->g.V;
-  double2 *work = (double2 *)workspace(ctx, "force_staples", sizeof(double2) * 9 * 16 * n);
+  const int64_t F3 = 27 * ctx->g.V;
+  const bool lepage = coef[4] != 0.0;
+  const int fields = lepage ? 18 : 12;
+  const Fat7Launch l = fat7_launch(ctx->g, fields);
+  double2 *work = (double2 *)workspace(ctx, "fat7", sizeof(double2) * l.nmu * l.per_mu);
   if (!work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (force staples)");
-  double2 *S3[3], *S5[3], *dS3[3], *dS5[3];
-  for (int i = 0; i < 3; i++) {
-    S3[i] = work + (size_t)(0 + i) * 9 * n;
-    S5[i] = work + (size_t)(3 + i) * 9 * n;
-    dS3[i] = work + (size_t)(6 + i) * 9 * n;
-    dS5[i] = work + (size_t)(9 + i) * 9 * n;
-  }
-  double2 *Pp = work + (size_t)12 * 9 * n, *Pm = work + (size_t)13 * 9 * n;
-  double2 *dPp = work + (size_t)14 * 9 * n, *dPm = work + (size_t)15 * 9 * n;
-  const Geom &g = ctx->g;
-  const unsigned grid = grid_for(n, kSmearThreads), ag = grid_for(9 * n, 256);
-  const double c1 = coef[0], c3 = coef[1], c5 = coef[2], c7 = coef[3], cL = coef[4];
-  for (int mu = 0; mu < 4; mu++) {
-    int axes[3], k = 0;
-    for (int d = 0; d < 4; d++)
-      if (d != mu) axes[k++] = d;
-    const double2 *Umu = U + (size_t)mu * 9 * n;
-    const double2 *dVmu = dV + (size_t)mu * 9 * n;
-    double2 *dUmu = dU + (size_t)mu * 9 * n;
-    // recompute the staples of this direction
-    for (int sl = 0; sl < 3; sl++)
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(S3[sl], Umu, U, g, mu, axes[sl], 3, 0, 1.0);
-    for (int sl = 0; sl < 3; sl++) {
-      const int bs = sl == 0 ? 1 : 0, cs = sl == 2 ? 1 : 2;
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(S5[sl], S3[cs], U, g, mu, axes[bs], 3, 0, 1.0);
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(S5[sl], S3[bs], U, g, mu, axes[cs], 3, 1, 1.0);
-    }
-    // seven-link terms c7 T_a(S5_a), and the five-link cotangents
-    for (int sl = 0; sl < 3; sl++) {
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dS5[sl], dVmu, U, g, mu, axes[sl], 3, 0, c7);
-      axpy_c_kernel<<<ag, 256, 0, st>>>(dS5[sl], dVmu, c5, 9 * n, 1);
-      transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dVmu, S5[sl], U, g, mu, axes[sl], 3, c7);
-    }
-    for (int sl = 0; sl < 3; sl++) axpy_c_kernel<<<ag, 256, 0, st>>>(dS3[sl], dVmu, c3, 9 * n, 0);
-    // five-link terms S5_a = T_b(S3_c) + T_c(S3_b)
-    for (int sl = 0; sl < 3; sl++) {
-      const int bs = sl == 0 ? 1 : 0, cs = sl == 2 ? 1 : 2;
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dS3[cs], dS5[sl], U, g, mu, axes[bs], 3, 1, 1.0);
-      transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dS5[sl], S3[cs], U, g, mu, axes[bs], 3, 1.0);
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dS3[bs], dS5[sl], U, g, mu, axes[cs], 3, 1, 1.0);
-      transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dS5[sl], S3[bs], U, g, mu, axes[cs], 3, 1.0);
-    }
-    // three-link terms S3_nu = T_nu(U_mu)
-    for (int sl = 0; sl < 3; sl++) {
-      staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dUmu, dS3[sl], U, g, mu, axes[sl], 3, 1, 1.0);
-      transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dS3[sl], Umu, U, g, mu, axes[sl], 3, 1.0);
-    }
-    axpy_c_kernel<<<ag, 256, 0, st>>>(dUmu, dVmu, c1, 9 * n, 1);
-    // Lepage: T+_nu(T+_nu(U_mu)) + T-_nu(T-_nu(U_mu)); the adjoint of T+ is T-
-    if (cL != 0.0) {
-      for (int sl = 0; sl < 3; sl++) {
-        const int nu = axes[sl];
-        staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(Pp, Umu, U, g, mu, nu, 1, 0, 1.0);
-        staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(Pm, Umu, U, g, mu, nu, 2, 0, 1.0);
-        staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dPp, dVmu, U, g, mu, nu, 2, 0, cL);
-        staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dPm, dVmu, U, g, mu, nu, 1, 0, cL);
-        transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dVmu, Pp, U, g, mu, nu, 1, cL);
-        transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dVmu, Pm, U, g, mu, nu, 2, cL);
-        staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dUmu, dPp, U, g, mu, nu, 2, 1, 1.0);
-        staple_transport_kernel<<<grid, kSmearThreads, 0, st>>>(dUmu, dPm, U, g, mu, nu, 1, 1, 1.0);
-        transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dPp, Umu, U, g, mu, nu, 1, 1.0);
-        transport_link_grad_kernel<<<grid, kSmearThreads, 0, st>>>(dU, dPm, Umu, U, g, mu, nu, 2, 1.0);
-      }
-    }
+  const Fat7Field fu{U, work, work + F3, lepage ? work + 4 * F3 : work + F3, 0.0};
+  const Fat7Field fg{dV, work + 2 * F3, work + 3 * F3, lepage ? work + 5 * F3 : work + 3 * F3, coef[1]};
+  for (int mu = 0; mu < 4; mu += l.nmu) {
+    if (lepage)
+      fat7_staples<2, true>(ctx, l, U, fu, fg, mu, coef, st);
+    else
+      fat7_staples<2, false>(ctx, l, U, fu, fg, mu, coef, st);
+    fat7_sum<true>(ctx, l, U, dU, fg, mu, coef[0], st);
+    Fat7Tiles tl;
+    const unsigned n = fat7_tiles(ctx->g, F7_GRAD, mu, 1, tl);
+    fat7_grad_kernel<<<4 * n, kFat7Threads, 0, st>>>(ctx->g, tl, U, dU, fu, fg, mu, l.nmu, l.per_mu, coef[3]);
   }
   LMB_CHECK_LAUNCH(ctx);
   return LMB_OK;
@@ -204,12 +230,12 @@ int clover_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_D
 }
 
 int accumulate_links_to(lmb_ctx *ctx, void *const dU[4], const double2 *planes, cudaStream_t st) {
-  const unsigned grid = grid_for(ctx->g.V, 256);
+  const unsigned grid = grid_for(ctx->g.V, kSmearThreads);
   if (ctx->dtype == LMB_DTYPE_C128)
-    accumulate_links_kernel<double2><<<grid, 256, 0, st>>>((double2 *)dU[0], (double2 *)dU[1], (double2 *)dU[2],
+    accumulate_links_kernel<double2><<<grid, kSmearThreads, 0, st>>>((double2 *)dU[0], (double2 *)dU[1], (double2 *)dU[2],
                                                             (double2 *)dU[3], planes, ctx->g, ctx->pd);
   else
-    accumulate_links_kernel<float2><<<grid, 256, 0, st>>>((float2 *)dU[0], (float2 *)dU[1], (float2 *)dU[2],
+    accumulate_links_kernel<float2><<<grid, kSmearThreads, 0, st>>>((float2 *)dU[0], (float2 *)dU[1], (float2 *)dU[2],
                                                            (float2 *)dU[3], planes, ctx->g, ctx->pd);
   LMB_CHECK_LAUNCH(ctx);
   return LMB_OK;
@@ -285,20 +311,20 @@ int lmb_hisq_links_from_thin(lmb_ctx *ctx, const void *const U[4], const uint64_
   const int64_t n = ctx->g.V;
   if (!same) {
     double2 *thin = (double2 *)workspace(ctx, "smear_thin", sizeof(double2) * 36 * n);
-    double2 *lvl1 = (double2 *)workspace(ctx, "smear_lvl1", sizeof(double2) * 36 * n);
     double2 *w = (double2 *)workspace(ctx, "smear_w", sizeof(double2) * 36 * n);
-    double2 *xo = (double2 *)workspace(ctx, "smear_out", sizeof(double2) * 36 * n);
-    if (!thin || !lvl1 || !w || !xo) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing)");
+    key.valid = false;  // the link sets are rewritten in place
+    double2 *fat = derived_planes(ctx, LMB_LINKS_FAT), *lng = derived_planes(ctx, LMB_LINKS_LONG);
+    if (!thin || !w || !fat || !lng) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing)");
     // hisq_links_from_thin! (HISQFullSmearing.jl:284-293)
     const double c_level1[5] = {1.0 / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, 0.0};
     const double c_level2[5] = {1.0 + naik_epsilon / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, -1.0 / 8};
     if ((rc = pack_links_to(ctx, thin, U, st))) return rc;
-    if ((rc = fat7_planes(ctx, thin, lvl1, c_level1, st))) return rc;
-    if ((rc = project_u3_planes(ctx, lvl1, w, st))) return rc;
-    if ((rc = fat7_planes(ctx, w, xo, c_level2, st))) return rc;
-    if ((rc = install_links(ctx, LMB_LINKS_FAT, xo, st))) return rc;
-    if ((rc = naik_planes(ctx, w, xo, st))) return rc;
-    if ((rc = install_links(ctx, LMB_LINKS_LONG, xo, st))) return rc;
+    if ((rc = fat7_planes(ctx, thin, lng, c_level1, st))) return rc;
+    if ((rc = project_u3_planes(ctx, lng, w, st))) return rc;
+    if ((rc = fat7_planes(ctx, w, fat, c_level2, st))) return rc;
+    if ((rc = naik_planes(ctx, w, lng, st))) return rc;
+    if ((rc = install_links(ctx, LMB_LINKS_FAT, st))) return rc;
+    if ((rc = install_links(ctx, LMB_LINKS_LONG, st))) return rc;
     for (int mu = 0; mu < 4; mu++) {
       key.ptr[mu] = U[mu];
       key.epoch[mu] = epoch ? epoch[mu] : 0;

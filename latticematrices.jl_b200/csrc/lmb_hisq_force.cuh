@@ -8,92 +8,13 @@
 // G_U = A^+ dT B^+ and, for a daggered occurrence A U^+ B, G_U = B dT^+ A.
 // Every kernel gathers the contributions to the site it owns (no atomics).
 //
-// Smearing levels are recomputed instead of stored: the Fat7 pullback of a
-// direction mu rebuilds that direction's 3- and 5-link staples from the
-// level's input links, then runs the factorised forward pass backwards.  The
-// staple transport
-//   T_nu(M)(x) = U_nu(x) M(x+nu) U_nu(x+mu)^+ + U_nu(x-nu)^+ M(x-nu) U_nu(x-nu+mu)
-// is its own adjoint in M (its forward half's adjoint is the backward half
-// and vice versa), so dM = T_nu(dT) reuses staple_transport_kernel.
+// Smearing levels are recomputed instead of stored; the Fat7 adjoint is in
+// lmb_fat7.cuh.
 #pragma once
 #include "lmb_hisq_smear.cuh"
 #include "lmb_staggered.cuh"
 
 namespace lmb {
-
-// dU_nu (+)= coef * d/dU_nu Re<dT, T_nu(M)> for the halves in `signs`
-// (1: U_nu(x) M(x+nu) U_nu(x+mu)^+, 2: U_nu(x-nu)^+ M(x-nu) U_nu(x-nu+mu))
-template <int = 0>
-__global__ void __launch_bounds__(kSmearThreads)
-    transport_link_grad_kernel(double2 *dUnu, const double2 *dT, const double2 *M, const double2 *U, const Geom g,
-                               int mu, int nu, int signs, double coef) {
-  const int z = blockIdx.x * kSmearThreads + threadIdx.x;
-  if (z >= g.V) return;
-  const int64_t V = g.V;
-  const double2 *Unu = U + (size_t)nu * 9 * V;
-  Cx<double> acc[9], a[9], b[9], c[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) acc[k] = Cx<double>(0, 0);
-  const int zpm = nb_site(g, z, mu, 1), zpn = nb_site(g, z, nu, 1), zmm = nb_site(g, z, mu, -1);
-  if (signs & 1) {
-    // (a) dT(z) U_nu(z+mu) M(z+nu)^+
-    load9(dT, V, z, a);
-    load9(Unu, V, zpm, b);
-    mat3_mul(a, b, a);
-    load9(M, V, zpn, c);
-    mat3_mul_adj(a, c, a);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + a[k];
-    // (b) dT(z-mu)^+ U_nu(z-mu) M(z-mu+nu)
-    const int zmm_pn = nb_site(g, zmm, nu, 1);
-    load9(dT, V, zmm, a);
-    load9(Unu, V, zmm, b);
-    mat3_adj_mul(a, b, a);
-    load9(M, V, zmm_pn, c);
-    mat3_mul(a, c, a);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + a[k];
-  }
-  if (signs & 2) {
-    // (c) M(z) U_nu(z+mu) dT(z+nu)^+
-    load9(M, V, z, a);
-    load9(Unu, V, zpm, b);
-    mat3_mul(a, b, a);
-    load9(dT, V, zpn, c);
-    mat3_mul_adj(a, c, a);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + a[k];
-    // (d) M(z-mu)^+ U_nu(z-mu) dT(z-mu+nu)
-    const int zmm_pn = nb_site(g, zmm, nu, 1);
-    load9(M, V, zmm, a);
-    load9(Unu, V, zmm, b);
-    mat3_adj_mul(a, b, a);
-    load9(dT, V, zmm_pn, c);
-    mat3_mul(a, c, a);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + a[k];
-  }
-  double2 *out = dUnu + (size_t)nu * 9 * V;
-  load9(out, V, z, b);
-#pragma unroll
-  for (int k = 0; k < 9; k++) b[k] = b[k] + coef * acc[k];
-  store9(out, V, z, b);
-}
-
-// y (+)= a x over n complex entries
-template <int = 0>
-__global__ void __launch_bounds__(256)
-    axpy_c_kernel(double2 *y, const double2 *x, double a, int64_t n, int accumulate) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const double2 v = x[i];
-  if (accumulate) {
-    const double2 w = y[i];
-    y[i] = make_double2(w.x + a * v.x, w.y + a * v.y);
-  } else {
-    y[i] = make_double2(a * v.x, a * v.y);
-  }
-}
 
 // Dirac outer products (HISQPullback.jl:461-513):
 //   dX_mu(x) = fc eta_mu(x) [dr(x) psi(x+mu)^+ - psi(x) dr(x+mu)^+]
@@ -271,24 +192,42 @@ __global__ void __launch_bounds__(64)
   store9(out, n, s, b);
 }
 
-// unpack-accumulate 36 gradient planes into four padded (3,3,...) fields
+// unpack-accumulate 36 gradient planes into four padded (3,3,...) fields.  The
+// fields hold a site's nine entries together, the planes a plane's sites: a
+// block of 128 sites turns one into the other through shared memory, so both
+// sides move whole lines (a thread per site left 16 of every 32 bytes of its
+// read-modify-write unused: 362 us at 24^4, 1.6 TB/s).
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kSmearThreads)
     accumulate_links_kernel(T *U0, T *U1, T *U2, T *U3, const double2 *src, const Geom g, const Padded pd) {
-  const int s = blockIdx.x * 256 + threadIdx.x;
-  if (s >= g.V) return;
-  int c[4];
-  site_coords(g, s, c);
-  const int64_t ps = padded_site(pd, c) * 9;
+  __shared__ double2 tile[9][kSmearThreads + 1];
+  __shared__ int64_t at[kSmearThreads];
+  const int s0 = blockIdx.x * kSmearThreads, t = threadIdx.x, s = s0 + t;
+  const int n = min(kSmearThreads, (int)(g.V - s0));
+  if (t < n) {
+    int c[4];
+    site_coords(g, s, c);
+    at[t] = padded_site(pd, c) * 9;
+  }
   T *U[4] = {U0, U1, U2, U3};
 #pragma unroll
-  for (int mu = 0; mu < 4; mu++)
+  for (int mu = 0; mu < 4; mu++) {
+    if (t < n) {
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-      const double2 t = src[(mu * 9 + k) * g.V + s];
-      U[mu][ps + k].x += t.x;
-      U[mu][ps + k].y += t.y;
+      for (int k = 0; k < 9; k++) tile[k][t] = src[(mu * 9 + k) * g.V + s];
     }
+    __syncthreads();
+    for (int i = t; i < 9 * n; i += kSmearThreads) {
+      const int site = i / 9, k = i - 9 * site;
+      const double2 v = tile[k][site];
+      T *u = U[mu] + at[site] + k;
+      T w = *u;
+      w.x += v.x;
+      w.y += v.y;
+      *u = w;
+    }
+    __syncthreads();
+  }
 }
 
 }  // namespace lmb

@@ -1,17 +1,8 @@
-// lmb_hisq_smear.cuh -- HISQ link smearing on the GPU (FP64).
+// lmb_hisq_smear.cuh -- 3x3 link algebra, U(3) projection and Naik links of the
+// HISQ smearing (FP64).
 //
-// Fat7 (+ Lepage) in the factorised form of the reference
-// (HISQSmearing.jl:768-974): for a link direction mu with transverse axes
-// (a, b, c) and the staple transport
-//   T_nu(M)(x) = U_nu(x) M(x+nu) U_nu(x+mu)^+ + U_nu(x-nu)^+ M(x-nu) U_nu(x-nu+mu),
-//   S3_nu = T_nu(U_mu),   S5_a = T_b(S3_c) + T_c(S3_b),
-//   V_mu = c1 U_mu + c3 sum S3 + c5 sum S5 + c7 sum_a T_a(S5_a) + cL Lepage,
-// which sums exactly the 6 three-link, 24 five-link and 48 seven-link paths of
-// the direct path lists (HISQSmearing.jl:490-566).  On one GPU every
-// intermediate field is defined on the whole periodic lattice, so no enlarged
-// domains are needed.  Lepage paths (nu,nu,mu,-nu,-nu), (-nu,-nu,mu,nu,nu)
-// are evaluated directly.  U(3) projection W = V (V^+V)^{-1/2} with the
-// trigonometric eigenvalues and Cayley-Hamilton coefficients
+// Fat7 (+ Lepage) lives in lmb_fat7.cuh.  U(3) projection W = V (V^+V)^{-1/2}
+// with the trigonometric eigenvalues and Cayley-Hamilton coefficients
 // (HISQFullSmearing.jl:1-77); Naik links L_mu(x) = W_mu(x) W_mu(x+mu) W_mu(x+2mu)
 // (HISQFullSmearing.jl:136-195).
 //
@@ -70,113 +61,6 @@ LMB_D int nb_site(const Geom &g, int s, int mu, int d) {
   int c[4], w;
   site_coords(g, s, c);
   return d > 0 ? fwd_site(g, s, c, mu, d, &w) : bwd_site(g, s, c, mu, -d, &w);
-}
-
-// out (+)= coef * T_nu(M) for link direction mu; signs: 1 forward, 2 backward, 3 both
-template <int = 0>
-__global__ void __launch_bounds__(kSmearThreads)
-    staple_transport_kernel(double2 *out, const double2 *M, const double2 *U, const Geom g, int mu, int nu,
-                            int signs, int accumulate, double coef) {
-  const int s = blockIdx.x * kSmearThreads + threadIdx.x;
-  if (s >= g.V) return;
-  const int64_t V = g.V;
-  Cx<double> acc[9], a[9], b[9], m[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) acc[k] = Cx<double>(0, 0);
-  if (signs & 1) {  // U_nu(x) M(x+nu) U_nu(x+mu)^+
-    const int xpn = nb_site(g, s, nu, 1), xpm = nb_site(g, s, mu, 1);
-    load9(U + (size_t)nu * 9 * V, V, s, a);
-    load9(M, V, xpn, m);
-    mat3_mul(a, m, a);
-    load9(U + (size_t)nu * 9 * V, V, xpm, b);
-    mat3_mul_adj(a, b, a);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + a[k];
-  }
-  if (signs & 2) {  // U_nu(x-nu)^+ M(x-nu) U_nu(x-nu+mu)
-    const int xmn = nb_site(g, s, nu, -1);
-    const int xmn_pm = nb_site(g, xmn, mu, 1);
-    load9(U + (size_t)nu * 9 * V, V, xmn, a);
-    load9(M, V, xmn, m);
-    mat3_adj_mul(a, m, a);
-    load9(U + (size_t)nu * 9 * V, V, xmn_pm, b);
-    mat3_mul(a, b, a);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + a[k];
-  }
-  if (accumulate) {
-    load9(out, V, s, m);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = m[k] + coef * acc[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = coef * acc[k];
-  }
-  store9(out, V, s, acc);
-}
-
-// V_mu = c1 U_mu + c3 (S3_a+S3_b+S3_c) + c5 (S5_a+S5_b+S5_c); fields single-direction
-template <int = 0>
-__global__ void __launch_bounds__(256)
-    fat7_combine_kernel(double2 *Vmu, const double2 *Umu, const double2 *s3a, const double2 *s3b,
-                        const double2 *s3c, const double2 *s5a, const double2 *s5b, const double2 *s5c, int64_t V,
-                        double c1, double c3, double c5) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= 9 * V) return;
-  const double2 u = Umu[i], a = s3a[i], b = s3b[i], c = s3c[i], d = s5a[i], e = s5b[i], f = s5c[i];
-  Vmu[i] = make_double2(c1 * u.x + c3 * (a.x + b.x + c.x) + c5 * (d.x + e.x + f.x),
-                        c1 * u.y + c3 * (a.y + b.y + c.y) + c5 * (d.y + e.y + f.y));
-}
-
-// product of links along a signed path (1-based directions) starting at s
-LMB_D void path_product_dev(const double2 *U, const Geom &g, int s, const int *path, int len, Cx<double> *out) {
-  const int64_t V = g.V;
-  Cx<double> m[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) out[k] = Cx<double>((k % 4) == 0 ? 1.0 : 0.0, 0);
-  int site = s;
-  for (int i = 0; i < len; i++) {
-    const int d = path[i];
-    const int axis = (d > 0 ? d : -d) - 1;
-    if (d > 0) {
-      load9(U + (size_t)axis * 9 * V, V, site, m);
-      mat3_mul(out, m, out);
-      site = nb_site(g, site, axis, 1);
-    } else {
-      site = nb_site(g, site, axis, -1);
-      load9(U + (size_t)axis * 9 * V, V, site, m);
-      mat3_mul_adj(out, m, out);
-    }
-  }
-}
-
-// V_mu += cL sum_nu [path(nu,nu,mu,-nu,-nu) + path(-nu,-nu,mu,nu,nu)]
-template <int = 0>
-__global__ void __launch_bounds__(kSmearThreads)
-    lepage_kernel(double2 *Vall, const double2 *U, const Geom g, double cL) {
-  const int64_t tid = (int64_t)blockIdx.x * kSmearThreads + threadIdx.x;
-  if (tid >= 4 * g.V) return;
-  const int mu = (int)(tid / g.V);
-  const int s = (int)(tid - (int64_t)mu * g.V);
-  Cx<double> acc[9], p[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) acc[k] = Cx<double>(0, 0);
-  for (int nu = 1; nu <= 4; nu++) {
-    if (nu == mu + 1) continue;
-    const int p1[5] = {nu, nu, mu + 1, -nu, -nu}, p2[5] = {-nu, -nu, mu + 1, nu, nu};
-    path_product_dev(U, g, s, p1, 5, p);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + p[k];
-    path_product_dev(U, g, s, p2, 5, p);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = acc[k] + p[k];
-  }
-  double2 *Vm = Vall + (size_t)mu * 9 * g.V;
-  Cx<double> v[9];
-  load9(Vm, g.V, s, v);
-#pragma unroll
-  for (int k = 0; k < 9; k++) v[k] = v[k] + cL * acc[k];
-  store9(Vm, g.V, s, v);
 }
 
 // (V^+V)^{-1/2} for the U(3) projection (HISQFullSmearing.jl:1-77):
@@ -256,6 +140,7 @@ __global__ void __launch_bounds__(kSmearThreads)
   store9(W + (size_t)mu * 9 * n, n, s, w);
 }
 
+// L_mu(x) = W_mu(x) W_mu(x+mu) W_mu(x+2mu)
 template <int = 0>
 __global__ void __launch_bounds__(kSmearThreads)
     naik_kernel(double2 *Lall, const double2 *W, const Geom g) {
@@ -263,10 +148,15 @@ __global__ void __launch_bounds__(kSmearThreads)
   if (t >= 4 * g.V) return;
   const int mu = (int)(t / g.V);
   const int s = (int)(t - (int64_t)mu * g.V);
-  const int path[3] = {mu + 1, mu + 1, mu + 1};
-  Cx<double> p[9];
-  path_product_dev(W, g, s, path, 3, p);
-  store9(Lall + (size_t)mu * 9 * g.V, g.V, s, p);
+  const double2 *Wm = W + (size_t)mu * 9 * g.V;
+  const int s1 = nb_site(g, s, mu, 1), s2 = nb_site(g, s1, mu, 1);
+  Cx<double> a[9], b[9];
+  load9(Wm, g.V, s, a);
+  load9(Wm, g.V, s1, b);
+  mat3_mul(a, b, a);
+  load9(Wm, g.V, s2, b);
+  mat3_mul(a, b, a);
+  store9(Lall + (size_t)mu * 9 * g.V, g.V, s, a);
 }
 
 // unpack 36 link planes to four padded (3,3,...) fields

@@ -1,0 +1,68 @@
+"""GPU: the kernels a size or storage rule selects, at the edges of their
+ranges.
+
+Bars: FP64 results against the oracle as the parity tests' (1e-13 relative
+norm; 1e-12 through the U(3) projection), FP32 5e-6, int16 2e-3 (one rounding
+of each operand per application); finite differences 1e-8 (step 1e-5: 1e-10
+truncation, 1e-11 rounding)."""
+import numpy as np
+import pytest
+
+import refdata as rd
+
+pytestmark = pytest.mark.gpu
+PHASES = (1, 1, 1, -1)
+TWISTED = tuple(np.exp(1j * a) for a in (0.13, -0.21, 0.34, np.pi - 0.17))
+
+
+@pytest.fixture(scope="module")
+def lmb():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import lmb200
+    lmb200.load()
+    return lmb200
+
+
+def _links(lmb, U, nw):
+    return [lmb.LatticeMatrix.from_array(u, nw=nw) for u in U]
+
+
+def _directions(L, seed):
+    rng = np.random.default_rng(seed)
+    return [np.asfortranarray(rng.normal(size=(3, 3) + L) + 1j * rng.normal(size=(3, 3) + L)) for _ in range(4)]
+
+
+# blocks of sites whose last ones are ragged in every extent; an extent below
+# the block's; one site more than a whole block
+@pytest.mark.parametrize("L", [(9, 5, 3, 7), (3, 4, 5, 4), (17, 3, 5, 3)])
+def test_fat7_levels_on_ragged_blocks(lmb, orc, L):
+    U = orc.random_su3_links(L, 0.25, 31)
+    fat, long = orc.hisq_links_from_thin(U, -0.083)
+    links = lmb.hisq_links_from_thin(_links(lmb, U, 3), -0.083)
+    for got, want in zip(links.fat_links + links.long_links, fat + long):
+        assert rd.rel_err(got.gather_matrix(), want) <= 1e-12
+
+
+# 4096 sites: four directions per launch; 17 x 16^3 = 69632 > 65536: one
+@pytest.mark.parametrize("L", [(9, 5, 3, 7), (8, 8, 8, 8), (17, 16, 16, 16)])
+def test_hisq_link_gradient_matches_finite_differences(lmb, orc, L):
+    eps, h = -0.083, 1e-5
+    U = orc.random_su3_links(L, 0.2, 41)
+    psi = lmb.LatticeMatrix.from_array(orc.gaussian_field(L, 3, 1, 42), nw=3, phases=PHASES)
+    chi = lmb.LatticeMatrix.from_array(orc.gaussian_field(L, 3, 1, 43), nw=3, phases=PHASES)
+    Ud = _links(lmb, U, 3)
+    cache = lmb.HISQDiracCache4D(Ud, 0.07, eps)
+    dU = [u.similar() for u in Ud]
+    lmb.hisq_link_pullback_(dU, cache, Ud, chi, psi)
+    V = _directions(L, 44)
+    out = psi.similar()
+
+    def loss(sign):
+        links = _links(lmb, [np.asfortranarray(u + sign * h * v) for u, v in zip(U, V)], 3)
+        lmb.mul_cached_hisq_(out, cache, *links, psi)
+        return lmb.dot(chi, out).real
+    fd = (loss(+1) - loss(-1)) / (2 * h)
+    an = sum(np.vdot(d.gather_matrix(), v).real for d, v in zip(dU, V))
+    assert abs(an - fd) <= 1e-8 * max(abs(fd), np.sqrt(np.prod(L)))
