@@ -208,7 +208,7 @@ int hisq_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_DOU
   return fat7_pullback_planes(ctx, thin, dV1, dU, c_level1, st);
 }
 
-// grad (36 planes) += d/dU [coef Re<dr, D_clover(U) psi>]
+// grad (36 planes) = d/dU [coef Re<dr, D_clover(U) psi>]
 int clover_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_DOUBLE, 12> &dr,
                            const Field<PREC_DOUBLE, 12> &psi, double kappa, double csw, double coefficient,
                            double2 *grad, cudaStream_t st) {
@@ -216,14 +216,20 @@ int clover_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_D
   wilson_outer_product_kernel<<<grid_for(n, 128), 128, 0, st>>>(grad, dr, psi, ctx->g, -kappa * coefficient);
   LMB_CHECK_LAUNCH(ctx);
   if (csw == 0.0) return LMB_OK;
-  double2 *dF = (double2 *)workspace(ctx, "force_dF", sizeof(double2) * 54 * n);
-  if (!dF) return fail(ctx, LMB_ERR_CUDA, "out of device memory (clover force)");
-  clover_cotangent_kernel<<<grid_for(n, 128), 128, 0, st>>>(dF, dr, psi, ctx->g, -kappa * csw * coefficient);
+  // the inserted links of all planes at once (1728 B per site), or of one
+  // plane at a time on lattices above 4 Mi sites: with the packed H that is
+  // less memory than the six full cotangents
+  const int np = n <= (1 << 22) ? 6 : 1;
+  double2 *H = (double2 *)workspace(ctx, "force_H", sizeof(double2) * 6 * kAntiPlanes * n);
+  double2 *W = (double2 *)workspace(ctx, "force_insert", sizeof(double2) * 18 * np * n);
+  if (!H || !W) return fail(ctx, LMB_ERR_CUDA, "out of device memory (clover force)");
+  clover_cotangent_kernel<<<grid_for(n, 128), 128, 0, st>>>(H, dr, psi, ctx->g, -kappa * csw * coefficient);
   LMB_CHECK_LAUNCH(ctx);
-  static const int pmu[6] = {0, 0, 0, 1, 1, 2}, pnu[6] = {1, 2, 3, 2, 3, 3};
-  for (int plane = 0; plane < 6; plane++) {
-    clover_link_pullback_kernel<<<grid_for(n, 64), 64, 0, st>>>(grad, thin, dF, ctx->g, plane, pmu[plane],
-                                                                 pnu[plane]);
+  Fat7Tiles tl;
+  const unsigned blocks = fat7_tiles(ctx->g, F7_SUM, 0, 4, tl);
+  for (int p = 0; p < 6; p += np) {
+    clover_insert_kernel<<<dim3(grid_for(n, kFat7Threads), 2 * np), kFat7Threads, 0, st>>>(W, thin, H, ctx->g, p);
+    clover_link_pullback_kernel<<<4 * blocks, kFat7Threads, 0, st>>>(grad, thin, W, ctx->g, tl, p, np);
     LMB_CHECK_LAUNCH(ctx);
   }
   return LMB_OK;
@@ -427,7 +433,6 @@ int lmb_wilson_clover_link_pullback(lmb_ctx *ctx, const void *const U[4], double
   if ((rc = pack_links_to(ctx, thin, U, st))) return rc;
   if ((rc = pack_in(ctx, dr, result_cotangent, st))) return rc;
   if ((rc = pack_in(ctx, ps, psi, st))) return rc;
-  LMB_CUDA(ctx, cudaMemsetAsync(grad, 0, sizeof(double2) * 36 * n, st));
   if ((rc = clover_pullback_planes(ctx, thin, dr, ps, kappa, csw, coefficient, grad, st))) return rc;
   return accumulate_links_to(ctx, dU, grad, st);
 }

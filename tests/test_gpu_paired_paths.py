@@ -66,3 +66,21 @@ def test_hisq_link_gradient_matches_finite_differences(lmb, orc, L):
     fd = (loss(+1) - loss(-1)) / (2 * h)
     an = sum(np.vdot(d.gather_matrix(), v).real for d, v in zip(dU, V))
     assert abs(an - fd) <= 1e-8 * max(abs(fd), np.sqrt(np.prod(L)))
+
+
+@pytest.mark.parametrize("L", [(9, 5, 3, 7), (4, 4, 6, 5)])
+def test_clover_link_gradient_on_odd_extents(lmb, orc, L):
+    kappa, csw, h = 0.13, 1.2, 1e-5
+    U = orc.random_su3_links(L, 0.2, 51)
+    psi, chi = orc.gaussian_field(L, 3, 4, 52), orc.gaussian_field(L, 3, 4, 53)
+    Ud = _links(lmb, U, 1)
+    D = lmb.WilsonDiracCloverOperator4D(Ud, kappa, csw)
+    dU = [u.similar() for u in Ud]
+    lmb.wilson_clover_link_pullback_(dU, D, Ud, lmb.LatticeMatrix.from_array(chi, nw=1, phases=TWISTED),
+                                     lmb.LatticeMatrix.from_array(psi, nw=1, phases=TWISTED))
+    V = _directions(L, 54)
+    loss = [np.vdot(chi, orc.wilson_clover([np.asfortranarray(u + s * h * v) for u, v in zip(U, V)], psi, kappa,
+                                           csw, TWISTED)).real for s in (+1, -1)]
+    fd = (loss[0] - loss[1]) / (2 * h)
+    an = sum(np.vdot(d.gather_matrix(), v).real for d, v in zip(dU, V))
+    assert abs(an - fd) <= 1e-8 * max(abs(fd), np.sqrt(np.prod(L)))
