@@ -1,6 +1,7 @@
 // lmb_op_dw.cuh -- domain-wall (5D) operator policy and its field hooks.
 #pragma once
 #include "lmb_domainwall.cuh"
+#include "lmb_domainwall_pair.cuh"
 #include "lmb_driver.cuh"
 
 namespace lmb {
@@ -18,6 +19,11 @@ struct DWPolicy {
     return ensure_link_precision(ctx, ctx->links[LMB_LINKS_THIN], prec, st);
   }
   static bool one_pass(const lmb_ctx *ctx) { return ctx->dw_L5 <= kDslashThreads && !ctx->dw_two_pass; }
+  // FP32 / int16: two slices per thread (every pair of slices is one 256-bit
+  // word of a plane when L5 is even)
+  static bool pairs(const lmb_ctx *ctx) {
+    return one_pass(ctx) && ctx->pair_sites && ctx->adj_sites && ctx->dw_L5 % 2 == 0;
+  }
   // blocks of the largest launch (the one-pass adjoint holds whole 4D points)
   static int64_t max_blocks(const lmb_ctx *ctx) {
     const int64_t flat = grid_for(ctx->g.V * ctx->dw_L5, kDslashThreads);
@@ -38,6 +44,19 @@ struct DWPolicy {
       return fail(ctx, LMB_ERR_CUDA, "out of device memory (domain-wall workspace)");
     const DWParams d = params(ctx);
     const unsigned grid = grid_for(V5, kDslashThreads);
+    if constexpr (P != PREC_DOUBLE) {
+      if (pairs(ctx)) {
+        const int half = d.L5 / 2;
+        if constexpr (!DAG) {
+          dw_forward_pair_kernel<<<grid_for(V4 * half, kDslashThreads), kDslashThreads, 0, st>>>(ctx->g, in, U, d, epi);
+        } else {
+          const int npts = kDslashThreads / half;
+          dw_adjoint_pair_kernel<<<grid_for(V4, npts), kDslashThreads, 0, st>>>(ctx->g, in, U, d, npts, epi);
+        }
+        LMB_CHECK_LAUNCH(ctx);
+        return LMB_OK;
+      }
+    }
     if (one_pass(ctx)) {
       if constexpr (!DAG) {
         dw_forward_kernel<R><<<grid, kDslashThreads, 0, st>>>(ctx->g, in, U, d, epi);

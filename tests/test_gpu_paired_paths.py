@@ -84,3 +84,23 @@ def test_clover_link_gradient_on_odd_extents(lmb, orc, L):
     fd = (loss[0] - loss[1]) / (2 * h)
     an = sum(np.vdot(d.gather_matrix(), v).real for d, v in zip(dU, V))
     assert abs(an - fd) <= 1e-8 * max(abs(fd), np.sqrt(np.prod(L)))
+
+
+# L5 = 2: a pair is its own neighbour on both sides; 128: the longest one-pass
+# fifth dimension; 6: blocks of the adjoint that leave threads idle
+@pytest.mark.parametrize("L5", [2, 6, 128])
+@pytest.mark.parametrize("precision,bar", [("single", 5e-6), ("half", 2e-3)])
+def test_domainwall_slice_pairs(lmb, orc, L5, precision, bar):
+    L = (3, 2, 4, 5) if L5 < 100 else (2, 2, 2, 3)
+    rng = np.random.default_rng(61)
+    U = orc.random_su3_links(L, 0.3, 62)
+    flat = orc.gaussian_field(L[:3] + (L[3] * L5,), 3, 4, 63)
+    psi = np.asfortranarray(flat.reshape((3, 4) + L + (L5,), order="F"))
+    a, b, c = (list(lo + w * rng.random(L5)) for lo, w in ((0.8, 0.4), (0.9, 0.6), (-0.3, 0.6)))
+    D = lmb.D5DW_GeneralizedDomainwallOperator5D(_links(lmb, U, 1), L5, 0.07, -1.8, a, b, c)
+    pd = lmb.LatticeMatrix.from_array(psi, 5, nw=1, phases=TWISTED + (1,))
+    out = pd.similar()
+    for dagger in (False, True):
+        lmb.mul_(out, lmb.adjoint(D) if dagger else D, pd, precision=precision)
+        ref = orc.domainwall(U, psi, 0.07, -1.8, a, b, c, TWISTED, dagger=dagger)
+        assert rd.rel_err(out.gather_matrix(), ref) <= bar
