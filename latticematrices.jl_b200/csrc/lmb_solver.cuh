@@ -332,6 +332,9 @@ struct EpiStoreFollow {
   template <typename R> LMB_D void operator()(int s, bool active, const Cx<R> *v) const {
     if (active) out.store(s, v);
   }
+  LMB_D void pair_adj(int s0, bool active, const Cx2 *v) const {
+    if (active) store_adj(out, s0, v);
+  }
 };
 
 // |b - v|^2 summed over the grid into *out (no CG state)

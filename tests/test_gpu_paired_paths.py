@@ -104,3 +104,21 @@ def test_domainwall_slice_pairs(lmb, orc, L5, precision, bar):
         lmb.mul_(out, lmb.adjoint(D) if dagger else D, pd, precision=precision)
         ref = orc.domainwall(U, psi, 0.07, -1.8, a, b, c, TWISTED, dagger=dagger)
         assert rd.rel_err(out.gather_matrix(), ref) <= bar
+
+
+# rows of 2 (one pair), 4 and 6 checkerboard sites take pairs; 3 one site per thread
+@pytest.mark.parametrize("L", [(4, 4, 2, 6), (8, 2, 4, 4), (12, 4, 2, 2), (6, 4, 2, 4)])
+@pytest.mark.parametrize("csw", [0.0, 1.0])
+def test_evenodd_pairs(lmb, orc, L, csw):
+    kappa = 0.125
+    U, b = orc.random_su3_links(L, 0.3, 71), orc.gaussian_field(L, 3, 4, 72)
+    Ud = _links(lmb, U, 1)
+    D = lmb.WilsonDiracCloverOperator4D(Ud, kappa, csw) if csw else lmb.WilsonDiracOperator4D(Ud, kappa)
+    bd = lmb.LatticeMatrix.from_array(b, nw=1, phases=TWISTED)
+    for precision in ("half", "single"):
+        x = bd.similar()
+        res = lmb.solve_evenodd_(x, D, bd, rtol=1e-10, precision=precision)
+        assert res.converged
+        xs = np.asfortranarray(x.gather_matrix())
+        Dx = orc.wilson_clover(U, xs, kappa, csw, TWISTED) if csw else orc.wilson(U, xs, kappa, TWISTED)
+        assert rd.rel_err(Dx, b) <= 1.05e-10
