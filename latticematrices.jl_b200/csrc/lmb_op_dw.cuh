@@ -89,6 +89,8 @@ struct DWPolicy {
 };
 
 inline int64_t op_volume(const lmb_ctx *ctx, const DWPolicy &) { return ctx->g.V * ctx->dw_L5; }
+template <> struct DirectOut<DWPolicy> { static constexpr bool value = true; };
+inline int op_slices(const lmb_ctx *ctx, const DWPolicy &) { return ctx->dw_L5; }
 inline int64_t op_max_blocks(const lmb_ctx *ctx, const DWPolicy &) { return DWPolicy::max_blocks(ctx); }
 template <int PS, int NC>
 int op_pack_in(lmb_ctx *ctx, const DWPolicy &, Field<PS, NC> &f, const void *src, cudaStream_t st) {

@@ -9,6 +9,8 @@ namespace lmb {
 // site_acc(s, active, v[3], red), then finish(red) once per block
 template <class Epi> struct PairSiteAcc { static constexpr bool value = false; };
 template <> struct PairSiteAcc<EpiStore<PREC_DOUBLE, 3>> { static constexpr bool value = true; };
+template <> struct PairSiteAcc<EpiStoreOut<3>> { static constexpr bool value = true; };
+template <int NC> struct StagMinBlocks<double, EpiStoreOut<NC>> { static constexpr int value = 5; };  // as EpiStore
 template <> struct PairSiteAcc<EpiStoreNorm<PREC_DOUBLE, 3>> { static constexpr bool value = true; };
 template <> struct PairSiteAcc<EpiCGUpdate<PREC_DOUBLE, PREC_DOUBLE, 3>> { static constexpr bool value = true; };
 
@@ -138,6 +140,8 @@ struct StaggeredPolicy {
     return ctx->links[LMB_LINKS_THIN].finite();
   }
 };
+
+template <> struct DirectOut<StaggeredPolicy> { static constexpr bool value = true; };
 
 LMB_OP_INSTANCES(extern, StaggeredPolicy)
 

@@ -98,6 +98,7 @@ struct WilsonPolicy {
   bool links_finite(const lmb_ctx *ctx) const { return ctx->links[LMB_LINKS_THIN].finite(); }
 };
 
+template <> struct DirectOut<WilsonPolicy> { static constexpr bool value = true; };
 LMB_OP_INSTANCES(extern, WilsonPolicy)
 
 }  // namespace lmb

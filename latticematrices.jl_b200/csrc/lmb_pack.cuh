@@ -32,7 +32,10 @@ __global__ void __launch_bounds__(256)
   typedef typename Real<PS>::type R;
   Cx<R> v[NC];
 #pragma unroll
-  for (int k = 0; k < NC; k++) v[k] = Cx<R>((R)q[k].x, (R)q[k].y);
+  for (int k = 0; k < NC; k++) {
+    const TIN t = q[k];  // whole (re, im) pairs: one 128-bit load
+    v[k] = Cx<R>((R)t.x, (R)t.y);
+  }
   dst.store(s, v);
 }
 
@@ -49,8 +52,10 @@ __global__ void __launch_bounds__(256)
   src.load(s, v);
 #pragma unroll
   for (int k = 0; k < NC; k++) {
-    q[k].x = v[k].re;
-    q[k].y = v[k].im;
+    TOUT t;  // whole (re, im) pairs: one 128-bit store
+    t.x = v[k].re;
+    t.y = v[k].im;
+    q[k] = t;
   }
 }
 

@@ -122,3 +122,40 @@ def test_evenodd_pairs(lmb, orc, L, csw):
         xs = np.asfortranarray(x.gather_matrix())
         Dx = orc.wilson_clover(U, xs, kappa, csw, TWISTED) if csw else orc.wilson(U, xs, kappa, TWISTED)
         assert rd.rel_err(Dx, b) <= 1.05e-10
+
+
+@pytest.mark.parametrize("L,nw,phases", [((3, 5, 4, 7), 1, TWISTED), ((8, 4, 4, 2), 0, PHASES), ((1, 1, 2, 3), 1, PHASES)])
+@pytest.mark.parametrize("scale", [1.0, 1.01])
+def test_fp64_wilson_small_and_odd(lmb, orc, L, nw, phases, scale):
+    """Reconstructed (scale 1) and 18-real links, extents down to 1."""
+    U = [np.asfortranarray(scale * u) for u in orc.random_su3_links(L, 0.3, 101)]
+    psi = orc.gaussian_field(L, 3, 4, 102)
+    Ud, pd = _links(lmb, U, nw), lmb.LatticeMatrix.from_array(psi, nw=nw, phases=phases)
+    out = pd.similar()
+    for csw in (0.0, 1.1):
+        D = lmb.WilsonDiracCloverOperator4D(Ud, 0.13, csw) if csw else lmb.WilsonDiracOperator4D(Ud, 0.13)
+        for dagger in (False, True):
+            lmb.mul_(out, lmb.adjoint(D) if dagger else D, pd)
+            ref = orc.wilson_clover(U, psi, 0.13, csw, phases, dagger=dagger) if csw else \
+                orc.wilson(U, psi, 0.13, phases, dagger=dagger)
+            assert rd.rel_err(out.gather_matrix(), ref) <= 1e-13
+
+
+def test_direct_store_leaves_the_halo_and_takes_any_alignment(lmb, orc):
+    """An output whose storage starts 16 bytes off a 32-byte boundary takes
+    128-bit stores; the ghosts stay as they were."""
+    import torch
+    L, nw = (4, 3, 5, 2), 1
+    U, psi = orc.random_su3_links(L, 0.3, 111), orc.gaussian_field(L, 3, 4, 112)
+    pd = lmb.LatticeMatrix.from_array(psi, nw=nw, phases=PHASES)
+    out = pd.similar()
+    shape = out.A.shape
+    store = torch.zeros(out.A.numel() + 1, dtype=out.A.dtype, device="cuda")
+    out.A = store[1:].view(shape)
+    out.A.fill_(7.0)
+    assert out.data_ptr() % 32 == 16
+    lmb.mul_(out, lmb.WilsonDiracOperator4D(_links(lmb, U, nw), 0.13), pd)
+    assert rd.rel_err(out.gather_matrix(), orc.wilson(U, psi, 0.13, PHASES)) <= 1e-13
+    ghosts = out.A.clone()
+    ghosts[1:-1, 1:-1, 1:-1, 1:-1] = 7.0
+    assert bool((ghosts == 7.0).all()) and complex(store[0]) == 0
