@@ -217,7 +217,7 @@ LMB_D void clover_apply(const C &A, int64_t s, Cx<R> *v) {
 //     + c2 (H in)(x)        (H^+ when DAG; in: parity 1 - p)
 //   out = A^-1(x) v when AINV, else v.     CL = false: A = 1.
 template <typename R, int DAG, int WMODE, bool AINV, bool CL, class SF, class G, class C, class Epi>
-__global__ void __launch_bounds__(kDslashThreads)
+__global__ void __launch_bounds__(kDslashThreads, SiteMinBlocks<R>::value)
     eo_hop_kernel(const Geom g, const int p, const SF in, const SF W, const G U, const C A, const C Ainv,
                   const R c1, const R c2, Epi epi) {
   if (epi.skip()) return;

@@ -36,6 +36,20 @@ namespace lmb {
 #endif
 constexpr int kDslashThreads = LMB_DSLASH_THREADS;
 
+// Resident blocks per SM of the one-site stencils.  The FP64 ones are bound by
+// the latency of their gathers and take 172 to 186 registers when left alone:
+// two blocks of 128 threads per SM.  Capped at three (168 registers, up to 80
+// bytes spilled): clover CG 24^3x48 254 -> 228 ms, Wilson CG 24^3x32 51.9 ->
+// 46.3 ms, even/odd clover 24^3x48 87.9 -> 77.8 ms, clover D and D^+ 24^4 274
+// -> 243 us; at four (128) 245, 49.1, 89.6 ms and 263 us.  (Two threads per
+// site, a colour vector of the half spinor each, at four blocks: 252 and
+// 54.6 ms.)
+#ifndef LMB_DSLASH_MINB_D
+#define LMB_DSLASH_MINB_D 3
+#endif
+template <typename R> struct SiteMinBlocks { static constexpr int value = LMB_DSLASH_MINB; };
+template <> struct SiteMinBlocks<double> { static constexpr int value = LMB_DSLASH_MINB_D; };
+
 // half-spin projection rows of (1 + PM g_mu) psi (WilsonDiracOperator.jl:157-175)
 template <int PM, int MU, typename R>
 LMB_D void project(const Cx<R> *p, Cx<R> *h) {
@@ -253,7 +267,7 @@ LMB_D void wilson_site_out(const Geom &g, int s, const int *c, const SF &in, con
 //   bool skip() const                      -- whole grid exits (paused solve)
 //   void operator()(s, active, out[12])    -- consume the result
 template <typename R, int DAG, bool CLOVER, int PHM, class SF, class G, class CL, class Epi>
-__global__ void __launch_bounds__(kDslashThreads, LMB_DSLASH_MINB)
+__global__ void __launch_bounds__(kDslashThreads, SiteMinBlocks<R>::value)
     wilson_dslash_kernel(const Geom g, const SF in, const G U, const CL A,
                          const R kappa, Epi epi, const SiteRange rg) {
   if (epi.skip()) return;
