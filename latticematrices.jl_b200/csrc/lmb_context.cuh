@@ -100,8 +100,9 @@ struct lmb_ctx {
   // (environment LMB_ADJ_SITES=0: sites s and s + V/2)
   bool adj_sites = true;
   // int16 K1 / K2 stencils as persistent kernels (one block per resident
-  // slot walking the tiles, one reduction per block); LMB_PERSISTENT=0 in
-  // the environment: one block per tile
+  // slot walking the tiles, one reduction per block), and the solves of small
+  // lattices as one cooperative launch (lmb_small.cuh); LMB_PERSISTENT=0 in
+  // the environment: one block per tile, one launch per CG stage
   bool persistent = true;
   // batched CG kernel family the autotuner may pick: -1 either, 0 links in
   // registers, 1 links in shared memory (environment LMB_BATCH_FAMILY)

@@ -26,6 +26,17 @@ int op_unpack_out(lmb_ctx *ctx, const Op &, void *dst, const Field<PS, NC> &f, c
   return unpack_out(ctx, dst, f, st);
 }
 
+// all iterations up to the next status change in one launch (lmb_small.cuh):
+// LMB_OK or an error; kNotSmall where the operator or the lattice has no such
+// kernel
+constexpr int kNotSmall = 1;
+constexpr int kSmallIters = 1000;
+template <class Op, int PS, int PX, int NC>
+int op_cg_small(lmb_ctx *, const Op &, const Field<PS, NC> &, const Field<PS, NC> &, const Field<PS, NC> &,
+                const Field<PX, NC> &, cudaStream_t) {
+  return kNotSmall;
+}
+
 // sites of an operator's fields in the caller's padded storage: 4D, or 5D
 // with L5 slices (site = slice + L5 x4, the slice slowest in the storage)
 struct PaddedOut {
@@ -321,7 +332,10 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
   EpiCGUpdate<PS, PX, NC> epi2{p, rl, xl, ctx->st_dev, ctx->partials, ctx->counter};
   while (hs->status == ST_RUNNING) {
     const int it0 = hs->iter;
-    for (int i = 0; i < k; i++) {
+    const int small = prm->profile ? kNotSmall : op_cg_small(ctx, op, p, rl, tl, xl, st);
+    if (small != kNotSmall && small != LMB_OK) return small;
+    if (small == LMB_OK) nl++;
+    for (int i = 0; i < k && small == kNotSmall; i++) {
       if (prm->profile) cudaEventRecord(pool.ev[4 * i], st);
       rc = op.template launch<PS, 0>(ctx, p, epi1, st);
       if (rc) return rc;
@@ -338,6 +352,8 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
     }
     rc = read_state(ctx, st);
     if (rc) return rc;
+    if (small == LMB_OK && hs->status == ST_RUNNING && hs->iter != it0 + kSmallIters)
+      return fail(ctx, LMB_ERR_CUDA, "a grid barrier of the small-lattice solver timed out");
     if (prm->profile) {
       const int real = hs->iter - it0 + (hs->status == ST_RELIABLE ? 1 : 0);
       for (int i = 0; i < real && i < k; i++) {

@@ -113,6 +113,11 @@ int op_unpack_out(lmb_ctx *ctx, const DWPolicy &, void *dst, const Field<PS, NC>
   return LMB_OK;
 }
 
+// small lattices (lmb_small_dw.cu)
+template <int PS, int PX>
+int op_cg_small(lmb_ctx *ctx, const DWPolicy &op, const Field<PS, 12> &p, const Field<PS, 12> &r,
+                const Field<PS, 12> &t, const Field<PX, 12> &x, cudaStream_t st);
+
 LMB_OP_INSTANCES(extern, DWPolicy)
 
 }  // namespace lmb

@@ -163,6 +163,11 @@ int evenodd_odd_g(lmb_ctx *ctx, const G &U, double kappa, const Field<PREC_DOUBL
 }
 
 
+// small lattices (lmb_small_schur.cu)
+template <int PS, int PX>
+int op_cg_small(lmb_ctx *ctx, const SchurPolicy &op, const Field<PS, 12> &p, const Field<PS, 12> &r,
+                const Field<PS, 12> &t, const Field<PX, 12> &x, cudaStream_t st);
+
 LMB_OP_INSTANCES(extern, SchurPolicy)
 
 }  // namespace lmb

@@ -143,6 +143,11 @@ struct StaggeredPolicy {
 
 template <> struct DirectOut<StaggeredPolicy> { static constexpr bool value = true; };
 
+// small lattices (lmb_small_staggered.cu)
+template <int PS, int PX>
+int op_cg_small(lmb_ctx *ctx, const StaggeredPolicy &op, const Field<PS, 3> &p, const Field<PS, 3> &r,
+                const Field<PS, 3> &t, const Field<PX, 3> &x, cudaStream_t st);
+
 LMB_OP_INSTANCES(extern, StaggeredPolicy)
 
 }  // namespace lmb

@@ -99,6 +99,11 @@ struct WilsonPolicy {
 };
 
 template <> struct DirectOut<WilsonPolicy> { static constexpr bool value = true; };
+// small lattices (lmb_small_wilson.cu)
+template <int PS, int PX>
+int op_cg_small(lmb_ctx *ctx, const WilsonPolicy &op, const Field<PS, 12> &p, const Field<PS, 12> &r,
+                const Field<PS, 12> &t, const Field<PX, 12> &x, cudaStream_t st);
+
 LMB_OP_INSTANCES(extern, WilsonPolicy)
 
 }  // namespace lmb

@@ -1,10 +1,12 @@
 """GPU: the kernels a size or storage rule selects, at the edges of their
-ranges.
+ranges: Fat7 on ragged site blocks and on both sides of the one-launch limit,
+the clover link gradient on odd extents, domain-wall slice pairs, even/odd
+pairs, the one-launch solver of small lattices, the two-lane FP64 Wilson
+stencil and the direct store of FP64 applications.
 
 Bars: FP64 results against the oracle as the parity tests' (1e-13 relative
-norm; 1e-12 through the U(3) projection), FP32 5e-6, int16 2e-3 (one rounding
-of each operand per application); finite differences 1e-8 (step 1e-5: 1e-10
-truncation, 1e-11 rounding)."""
+norm), FP32 5e-6, int16 2e-3 (one rounding of each operand per application);
+finite differences 1e-8 (step 1e-5: 1e-10 truncation, 1e-11 rounding)."""
 import numpy as np
 import pytest
 
@@ -122,6 +124,83 @@ def test_evenodd_pairs(lmb, orc, L, csw):
         xs = np.asfortranarray(x.gather_matrix())
         Dx = orc.wilson_clover(U, xs, kappa, csw, TWISTED) if csw else orc.wilson(U, xs, kappa, TWISTED)
         assert rd.rel_err(Dx, b) <= 1.05e-10
+
+
+def _solver(lmb, orc, op, L, scale, precision, phases):
+    """A solve of `op` on a new context: (result, solution)."""
+    U = [np.asfortranarray(scale * u) for u in orc.random_su3_links(L, 0.25, 81)]
+    nw, spins = (3 if op == "hisq" else 1), (1 if op in ("staggered", "hisq") else 4)
+    Ud = _links(lmb, U, nw)
+    if op == "domainwall":
+        flat = orc.gaussian_field(L[:3] + (L[3] * 5,), 3, 4, 82)
+        b = lmb.LatticeMatrix.from_array(np.asfortranarray(flat.reshape((3, 4) + L + (5,), order="F")), 5, nw=1,
+                                         phases=phases + (1,))
+        D = lmb.D5DW_MobiusDomainwallOperator5D(Ud, 5, 0.2, -1.4, 1.5, 0.5)
+    else:
+        b = lmb.LatticeMatrix.from_array(orc.gaussian_field(L, 3, spins, 82), nw=nw, phases=phases)
+        D = {"wilson": lambda: lmb.WilsonDiracOperator4D(Ud, 0.12),
+             "clover": lambda: lmb.WilsonDiracCloverOperator4D(Ud, 0.12, 1.0),
+             "evenodd": lambda: lmb.WilsonDiracOperator4D(Ud, 0.12),
+             "evenodd-clover": lambda: lmb.WilsonDiracCloverOperator4D(Ud, 0.12, 1.0),
+             "staggered": lambda: lmb.StaggeredDiracOperator4D(Ud, 0.2),
+             "hisq": lambda: lmb.HISQDiracCache4D(Ud, 0.2, -0.083)}[op]()
+    x = b.similar()
+    if op.startswith("evenodd"):
+        res = lmb.solve_evenodd_(x, D, b, rtol=1e-9, maxiter=400, precision=precision)
+    else:
+        res = lmb.cg_(x, lmb.DdagDOp(D, b.similar()), b, rtol=1e-9, maxiter=400, precision=precision)
+    return res, x.gather_matrix()
+
+
+# the one-launch solver against one launch per stage (LMB_PERSISTENT=0): a
+# lattice below one tile of 32 sites per block, ragged last tiles, links that
+# are not SU(3) (18 reals)
+@pytest.mark.parametrize("op", ["wilson", "clover", "staggered", "hisq", "evenodd", "evenodd-clover", "domainwall"])
+@pytest.mark.parametrize("L,scale", [((3, 3, 3, 4), 1.0), ((5, 3, 7, 6), 1.0), ((4, 6, 4, 8), 1.01)])
+@pytest.mark.parametrize("precision", ["double", "single", "half"])
+def test_small_lattice_solver(lmb, orc, monkeypatch, op, L, scale, precision):
+    if op in ("staggered", "hisq") or op.startswith("evenodd"):  # even extents: signs, parity
+        L = {(3, 3, 3, 4): (4, 4, 4, 4), (5, 3, 7, 6): (6, 6, 6, 6)}.get(L, L)
+    out = []
+    for stages in ("1", "0"):
+        monkeypatch.setenv("LMB_PERSISTENT", stages)
+        out.append(_solver(lmb, orc, op, L, scale, precision, TWISTED))
+    (ra, xa), (rb, xb) = out
+    assert ra.reason == rb.reason
+    assert abs(ra.iterations - rb.iterations) <= (1 if precision == "double" else max(3, rb.iterations // 20))
+    if ra.converged:  # both within 1e-9 of the same equation
+        assert rd.rel_err(xa, xb) <= 1e-6
+
+
+def test_small_lattice_solver_stops_as_the_staged_one(lmb, orc, monkeypatch):
+    L = (4, 4, 4, 4)
+    U = orc.random_su3_links(L, 0.3, 91)
+    b = lmb.LatticeMatrix.from_array(orc.gaussian_field(L, 3, 4, 92), nw=1, phases=PHASES)
+    for precision in ("double", "half"):
+        for maxiter in (0, 1, 7):
+            got = []
+            for stages in ("1", "0"):
+                monkeypatch.setenv("LMB_PERSISTENT", stages)
+                D = lmb.WilsonDiracOperator4D(_links(lmb, U, 1), 0.12)
+                res = lmb.cg_(b.similar(), lmb.DdagDOp(D, b.similar()), b, maxiter=maxiter, precision=precision)
+                got.append((res.reason, res.iterations))
+                assert res.iterations <= maxiter
+            assert got[0] == got[1] == ("maximum_iterations", maxiter)
+
+
+# FP64: the one launch up to 4 tiles per resident block, 37888 sites on 148 SMs
+@pytest.mark.parametrize("L", [(16, 16, 12, 12), (16, 16, 12, 14)])
+def test_solvers_on_both_sides_of_the_limit(lmb, orc, L):
+    U = lmb.random_su3_links(L, 0.25, 95)
+    b = lmb.gaussian_fermion(L, 3, 4, 96, phases=PHASES)
+    D = lmb.WilsonDiracOperator4D(U, 0.12)
+    for precision in ("double", "half"):
+        x = b.similar()
+        res = lmb.cg_(x, lmb.DdagDOp(D, b.similar()), b, rtol=1e-10, precision=precision)
+        t, y = b.similar(), b.similar()
+        lmb.DdagDOp(D, t).mul_(y, x)
+        r = (y.core_view() - b.core_view()).norm() / b.core_view().norm()
+        assert res.converged and float(r) <= 1.1e-10
 
 
 @pytest.mark.parametrize("L,nw,phases", [((3, 5, 4, 7), 1, TWISTED), ((8, 4, 4, 2), 0, PHASES), ((1, 1, 2, 3), 1, PHASES)])
