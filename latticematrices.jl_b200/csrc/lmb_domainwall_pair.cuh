@@ -13,12 +13,13 @@
 //
 // What bounds it: issue and latency, not DRAM (int16 D5 has 112 B per site to
 // move, 27 us at 16^3x32x12; its packed arithmetic alone takes about 85 us).
-// At that size a D5 takes 197 us on int16 fields (one site per thread: 242)
-// and a D5^+ with the CG update 189 (231); the solves take 223 ms on int16
-// (265) and 273 ms on FP32 fields (290).  Three blocks of 168 registers; two
-// of 255 and four of 128 (spilling) measured 247 and 221 ms on int16, 281 and
-// 286 ms on FP32.  FP32 links of 18 reals for int16 fields, which spare the
-// decode and the third row, measured slower (241 ms).
+// At that size a D5 takes 195 us on int16 fields (one site per thread: 242)
+// and a D5^+ with the CG update 178 (231); the solves take 217 ms on int16
+// (265) and 262 ms on FP32 fields (290).  The other way round, int16 on three
+// blocks of 168 registers and FP32 on four of 128, they take 223 and 284 ms;
+// with the link in both lanes of 36 registers 223 and 269 ms on three blocks.
+// FP32 links of 18 reals for int16 fields, which spare the decode and the third
+// row, measured slower (241 ms).
 #pragma once
 #include "lmb_domainwall.cuh"
 #include "lmb_pair_hop.cuh"
@@ -32,6 +33,11 @@ LMB_D float2 dw_lanes(const double *v, int s0, int s1, double f0, double f1) {
 // (lo.x from q, lo.y from lane x of p) and (hi.x from lane y of p, hi.y from q)
 LMB_D Cx2 dw_below(const Cx<float> &q, const Cx2 &p) { return Cx2(f2(q.re, p.re.x), f2(q.im, p.im.x)); }
 LMB_D Cx2 dw_above(const Cx2 &p, const Cx<float> &q) { return Cx2(f2(p.re.y, q.re), f2(p.im.y, q.im)); }
+
+// resident blocks per SM: int16 words leave room for four (128 registers, D5
+// spills 170 bytes), FP32 ones for three
+template <class SF> struct DWPairBlocks { static constexpr int value = 3; };
+template <> struct DWPairBlocks<Field<PREC_HALF, 12>> { static constexpr int value = 4; };
 
 // slices and coefficients of a pair: i0 = index of slice s within the point,
 // below / above the slices next to the pair, and for D5 the factors of
@@ -65,12 +71,48 @@ LMB_D void dw_Y_proj2(const SF &psi, int64_t base, const DWPair &d, Cx2 *h) {
   for (int k = 0; k < 6; k++) h[k] = Cx2(fma2(d.ch, t[k].re, h[k].re), fma2(d.ch, t[k].im, h[k].im));
 }
 
+// one link for both lanes, U h and U^+ h: an entry is put into both lanes where
+// it is used, for the two colour vectors at once, so that the link takes 18
+// registers and not 36
+LMB_D void shared_mul_half(const Cx<float> *u, const Cx2 *h, Cx2 *o) {
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const Cx2 e(f2(u[r].re), f2(u[r].im));
+    o[r] = e * h[0];
+    o[r + 3] = e * h[3];
+  }
+#pragma unroll
+  for (int k = 1; k < 3; k++)
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const Cx2 e(f2(u[r + 3 * k].re), f2(u[r + 3 * k].im));
+      o[r] = cfma(e, h[k], o[r]);
+      o[r + 3] = cfma(e, h[k + 3], o[r + 3]);
+    }
+}
+LMB_D void shared_adj_mul_half(const Cx<float> *u, const Cx2 *h, Cx2 *o) {
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const Cx2 e(f2(u[3 * r].re), f2(-u[3 * r].im));
+    o[r] = e * h[0];
+    o[r + 3] = e * h[3];
+  }
+#pragma unroll
+  for (int k = 1; k < 3; k++)
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const Cx2 e(f2(u[3 * r + k].re), f2(u[3 * r + k].im));
+      o[r] = cfma_conj(e, h[k], o[r]);
+      o[r + 3] = cfma_conj(e, h[k + 3], o[r + 3]);
+    }
+}
+
 template <int DAG, int MU, bool FUSED, class SF, class G>
 LMB_D void dw_hop2(const Geom &g, int x4, const int *c, int L5, const DWPair &d, const SF &in, const G &U,
                    Cx2 *acc) {
   constexpr int FPM = DAG ? +1 : -1;
   constexpr int BPM = -FPM;
-  Cx2 h[6], uh[6], u[9];
+  Cx2 h[6], uh[6];
   Cx<float> us[9];
   int wrap;
   {
@@ -82,9 +124,7 @@ LMB_D void dw_hop2(const Geom &g, int x4, const int *c, int L5, const DWPair &d,
     }
     if (wrap && ((g.phase_mask >> MU) & 1)) phase2(h, g.ph_fwd[MU], 1, 1);
     U.load(MU, x4, us);
-#pragma unroll
-    for (int k = 0; k < 9; k++) u[k] = Cx2(f2(us[k].re), f2(us[k].im));
-    su3_mul_half(u, h, uh);
+    shared_mul_half(us, h, uh);
     reconstruct<FPM, MU>(acc, uh);
   }
   {
@@ -96,9 +136,7 @@ LMB_D void dw_hop2(const Geom &g, int x4, const int *c, int L5, const DWPair &d,
     }
     if (wrap && ((g.phase_mask >> MU) & 1)) phase2(h, g.ph_bwd[MU], 1, 1);
     U.load(MU, sm, us);
-#pragma unroll
-    for (int k = 0; k < 9; k++) u[k] = Cx2(f2(us[k].re), f2(us[k].im));
-    su3_adj_mul_half(u, h, uh);
+    shared_adj_mul_half(us, h, uh);
     reconstruct<BPM, MU>(acc, uh);
   }
 }
@@ -125,7 +163,7 @@ LMB_D DWPair dw_pair(int s, int L5) {
 
 // D5: one thread per pair of slices
 template <class SF, class G, class Epi>
-__global__ void __launch_bounds__(kDslashThreads, 3)
+__global__ void __launch_bounds__(kDslashThreads, DWPairBlocks<SF>::value)
     dw_forward_pair_kernel(const Geom g, const SF psi, const G U, const DWParams dw, Epi epi) {
   if (epi.skip()) return;
   const int L5 = dw.L5, half = L5 / 2;
@@ -166,7 +204,7 @@ __global__ void __launch_bounds__(kDslashThreads, 3)
 
 // D5^+: blocks of `npts` whole 4D points (npts * L5 / 2 <= kDslashThreads)
 template <class SF, class G, class Epi>
-__global__ void __launch_bounds__(kDslashThreads, 3)
+__global__ void __launch_bounds__(kDslashThreads, DWPairBlocks<SF>::value)
     dw_adjoint_pair_kernel(const Geom g, const SF psi, const G U, const DWParams dw, int npts, Epi epi) {
   // of every pair, what its neighbours take: spins 1, 2 of lane x (the pair
   // below it) and spins 3, 4 of lane y (the pair above)
