@@ -30,6 +30,12 @@ unsigned resident_grid(const lmb_ctx *ctx, K kern) {
   return (unsigned)(resident_blocks_per_sm((const void *)kern) * (ctx->sm_count > 0 ? ctx->sm_count : 1));
 }
 
+// whether `threads` threads of a pair kernel (three blocks of 128 per SM) fill at
+// least num / den of the device's resident blocks
+inline bool fills_device(const lmb_ctx *ctx, int64_t threads, int num, int den) {
+  return den * threads >= (int64_t)num * 3 * kDslashThreads * (ctx->sm_count > 0 ? ctx->sm_count : 1);
+}
+
 inline int check_prec(lmb_ctx *ctx, int prec) {
   if (prec < PREC_DOUBLE || prec > PREC_HALF) return fail(ctx, LMB_ERR_ARG, "unknown precision %d", prec);
   return LMB_OK;

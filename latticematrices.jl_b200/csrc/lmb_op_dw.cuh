@@ -20,9 +20,15 @@ struct DWPolicy {
   }
   static bool one_pass(const lmb_ctx *ctx) { return ctx->dw_L5 <= kDslashThreads && !ctx->dw_two_pass; }
   // FP32 / int16: two slices per thread (every pair of slices is one 256-bit
-  // word of a plane when L5 is even)
-  static bool pairs(const lmb_ctx *ctx) {
-    return one_pass(ctx) && ctx->pair_sites && ctx->adj_sites && ctx->dw_L5 % 2 == 0;
+  // word of a plane when L5 is even), on lattices that give the half as many
+  // threads enough blocks.  Solves, one site -> pairs: int16 8^3x12x8 (192
+  // blocks of 444) 11.0 -> 11.1 ms, 8^3x16x8 (256) 14.5 -> 13.8, 12^3x16^2
+  // (864) 55.7 -> 47.1; FP32 8^3x16x8 14.1 -> 15.4, 8^2x12^2x10 (360) 17.7 ->
+  // 15.8, 8^2x12x16x12 (576, two waves) 24.9 -> 25.6, 8x12^2x16x12 (864) 33.0
+  // -> 30.0.
+  template <int P> static bool pairs(const lmb_ctx *ctx) {
+    return one_pass(ctx) && ctx->pair_sites && ctx->adj_sites && ctx->dw_L5 % 2 == 0 &&
+           fills_device(ctx, ctx->g.V * (ctx->dw_L5 / 2), P == PREC_HALF ? 2 : 3, 4);
   }
   // blocks of the largest launch (the one-pass adjoint holds whole 4D points)
   static int64_t max_blocks(const lmb_ctx *ctx) {
@@ -45,7 +51,7 @@ struct DWPolicy {
     const DWParams d = params(ctx);
     const unsigned grid = grid_for(V5, kDslashThreads);
     if constexpr (P != PREC_DOUBLE) {
-      if (pairs(ctx)) {
+      if (pairs<P>(ctx)) {
         const int half = d.L5 / 2;
         if constexpr (!DAG) {
           dw_forward_pair_kernel<<<grid_for(V4 * half, kDslashThreads), kDslashThreads, 0, st>>>(ctx->g, in, U, d, epi);

@@ -87,8 +87,10 @@ struct SchurPolicy {
       // pairs of checkerboard neighbours stay in one row when the row holds
       // an even number of them.  int16 only: at 24^3x48 clover its solve takes
       // 35.3 ms on pairs against 40.2 ms, the FP32 one, whose loads already
-      // fill the registers, 53.6 against 50.5 ms
-      if (ctx->pair_sites && ctx->adj_sites && ctx->g.L[0] % 4 == 0) {
+      // fill the registers, 53.6 against 50.5 ms.  And from half the resident
+      // blocks on: clover 16^4 (128 blocks of 444) 6.3 -> 6.6 ms, 16^2x24^2
+      // (288) 10.4 -> 9.8
+      if (ctx->pair_sites && ctx->adj_sites && ctx->g.L[0] % 4 == 0 && fills_device(ctx, ctx->g.V / 4, 1, 2)) {
         const unsigned g2 = grid_for(ctx->g.V / 4, kDslashThreads);
         eo_hop_pair_kernel<DAG, 0, true, CL><<<g2, kDslashThreads, 0, st>>>(ctx->g, 1, in, in, U, A, Ai, 0.f, 1.f, e1);
         eo_hop_pair_kernel<DAG, 2, false, CL><<<g2, kDslashThreads, 0, st>>>(ctx->g, 0, t, in, U, A, Ai, 1.f,

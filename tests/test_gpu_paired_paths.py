@@ -88,12 +88,13 @@ def test_clover_link_gradient_on_odd_extents(lmb, orc, L):
     assert abs(an - fd) <= 1e-8 * max(abs(fd), np.sqrt(np.prod(L)))
 
 
-# L5 = 2: a pair is its own neighbour on both sides; 128: the longest one-pass
-# fifth dimension; 6: blocks of the adjoint that leave threads idle
-@pytest.mark.parametrize("L5", [2, 6, 128])
+# lattices of at least 222 (int16) and 333 (FP32) blocks of 128 pairs, which
+# take them on 148 SMs.  L5 = 2: a pair is its own neighbour on both sides; 128:
+# the longest one-pass fifth dimension; 6: blocks of the adjoint that leave
+# threads idle
+@pytest.mark.parametrize("L,L5", [((15, 16, 14, 13), 2), ((11, 12, 10, 11), 6), ((6, 5, 6, 5), 128)])
 @pytest.mark.parametrize("precision,bar", [("single", 5e-6), ("half", 2e-3)])
-def test_domainwall_slice_pairs(lmb, orc, L5, precision, bar):
-    L = (3, 2, 4, 5) if L5 < 100 else (2, 2, 2, 3)
+def test_domainwall_slice_pairs(lmb, orc, L, L5, precision, bar):
     rng = np.random.default_rng(61)
     U = orc.random_su3_links(L, 0.3, 62)
     flat = orc.gaussian_field(L[:3] + (L[3] * L5,), 3, 4, 63)
@@ -108,11 +109,13 @@ def test_domainwall_slice_pairs(lmb, orc, L5, precision, bar):
         assert rd.rel_err(out.gather_matrix(), ref) <= bar
 
 
-# rows of 2 (one pair), 4 and 6 checkerboard sites take pairs; 3 one site per thread
-@pytest.mark.parametrize("L", [(4, 4, 2, 6), (8, 2, 4, 4), (12, 4, 2, 2), (6, 4, 2, 4)])
+# from 222 blocks of 128 pairs on (113664 sites on 148 SMs) rows of 2 (one pair),
+# 4 and 12 checkerboard sites take pairs; a row of 3 or 9 stays at one site per
+# thread, and so do the small ones
+@pytest.mark.parametrize("L", [(4, 32, 30, 32), (8, 30, 20, 24), (24, 18, 16, 18), (18, 18, 20, 18), (6, 4, 2, 4)])
 @pytest.mark.parametrize("csw", [0.0, 1.0])
 def test_evenodd_pairs(lmb, orc, L, csw):
-    kappa = 0.125
+    kappa = 0.115
     U, b = orc.random_su3_links(L, 0.3, 71), orc.gaussian_field(L, 3, 4, 72)
     Ud = _links(lmb, U, 1)
     D = lmb.WilsonDiracCloverOperator4D(Ud, kappa, csw) if csw else lmb.WilsonDiracOperator4D(Ud, kappa)
