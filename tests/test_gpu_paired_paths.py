@@ -1,8 +1,8 @@
 """GPU: the kernels a size or storage rule selects, at the edges of their
 ranges: Fat7 on ragged site blocks and on both sides of the one-launch limit,
 the clover link gradient on odd extents, domain-wall slice pairs, even/odd
-pairs, the one-launch solver of small lattices, the two-lane FP64 Wilson
-stencil and the direct store of FP64 applications.
+pairs, the one-launch solver of small lattices and the direct store of FP64
+applications.
 
 Bars: FP64 results against the oracle as the parity tests' (1e-13 relative
 norm), FP32 5e-6, int16 2e-3 (one rounding of each operand per application);
