@@ -48,6 +48,8 @@ FP64_ITERATIONS_32x64 = 450
 #  K1  tmp = D p  (+|tmp|^2):  links, clover, p, tmp
 #  K2  D^+ tmp fused with x += a p, r -= a Ap, |r|^2:  links, clover, tmp,
 #      p, r (read+write), x (read+write, FP32 for the mixed solves)
+#      (x once in X_UPDATE iterations, for all of them)
+X_UPDATE = 4
 REAL_BYTES = {"double": 8, "single": 4, "half": 2}
 
 
@@ -68,7 +70,7 @@ def k1_bytes(prec, link_reals=18):
 
 
 def k2_bytes(prec, link_reals=18):
-    return gauge_bytes(prec, link_reals) + 4 * spinor_bytes(prec) + 2 * x_bytes(prec)
+    return gauge_bytes(prec, link_reals) + 4 * spinor_bytes(prec) + 2 * x_bytes(prec) // X_UPDATE
 
 
 # Wilson-clover M: 1320 (hopping) + 504 (clover) + 48 flops per site
@@ -614,11 +616,11 @@ def run_hisq(args):
     out = {"workload": "HISQ smearing + staggered D'D CG, %dx%dx%dx%d, m 0.01" % L,
            "smear_s": t_smear}
     # algorithmic bytes per site (each link matrix once: 4 fat + 4 Naik x 18
-    # reals; K1 links + in + out, K2 links + in + p + r (rw) + x (rw)):
-    # FP32 / FP64 156 and 180 reals; int16 links 8 x 36 B, spinor 16 B + 4 B
-    # norm, x FP32 24 B
-    kbytes = {"single": (156 * 4, 180 * 4), "double": (156 * 8, 180 * 8),
-              "half": (288 + 2 * 20, 288 + 4 * 20 + 2 * 24)}
+    # reals; K1 links + in + out, K2 links + in + p + r (rw) + x (rw, once in
+    # X_UPDATE iterations)): FP32 / FP64 156 and 171 reals; int16 links
+    # 8 x 36 B, spinor 16 B + 4 B norm, x FP32 24 B
+    kbytes = {"single": (156 * 4, 171 * 4), "double": (156 * 8, 171 * 8),
+              "half": (288 + 2 * 20, 288 + 4 * 20 + 2 * 24 // X_UPDATE)}
     for prec in ("single", "half", "double"):
         lmb.clear_matrix_(x)
         lmb.cg_(x, A, b, rtol=1e-10, precision=prec, maxiter=args.maxiter)
@@ -938,12 +940,12 @@ def run_dw(args):
         # bytes per 5D site the two-pass kernels move (each operand once):
         #  K1 = D5 p:  Y = B p + C F p (p, Y), stencil (Y, p, out, links)
         #  K2 = D5^+ t + CG update: stencil (t, Z, links), local (t, Z, p,
-        #       r rw, x rw)
+        #       r rw, x rw once in X_UPDATE iterations)
         k1_b = 5 * sp + links
-        k2_b = 7 * sp + 2 * xb + links
+        k2_b = 7 * sp + 2 * xb // X_UPDATE + links
         # the operator's compulsory bytes (a one-pass kernel): in, out, links
         k1_min = 2 * sp + links
-        k2_min = 4 * sp + 2 * xb + links
+        k2_min = 4 * sp + 2 * xb // X_UPDATE + links
         out[prec] = {"time_s": t, "iterations": res.iterations, "converged": res.converged,
                      "true_rel_residual": res.true_residual_norm / bn,
                      "reliable_updates": res.reliable_updates,

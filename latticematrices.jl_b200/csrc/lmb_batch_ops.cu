@@ -511,7 +511,7 @@ int cg_batched(lmb_ctx *ctx, const lmb_cg_params *prm, int nlat, const lmb_batch
           if ((masks[gi] >> r) & 1) {
             BatchMember<PS> &mm = m[aux.groups[gi].state0 + r];
             cg_p_update_kernel<PS, 12><<<grid_for(mm.g.V, kBlasThreads), kBlasThreads, 0, st>>>(
-                mm.p, mm.r, states + aux.groups[gi].state0 + r, mm.g.V);
+                mm.p, mm.p, mm.r, states + aux.groups[gi].state0 + r, mm.g.V);
           }
       LMB_CHECK_LAUNCH(ctx);
       if ((rc = read_all())) { cleanup(); return rc; }

@@ -205,17 +205,18 @@ struct EventPool {
   }
 };
 
-// K3: p = r + beta p; FP32 / int16 Wilson fields of an even volume use the
+// K3: pn = r + beta p (pn may be p); FP32 / int16 Wilson fields of an even volume use the
 // two-site kernel (256-bit accesses)
 template <int PS, int NC>
-void launch_p_update(lmb_ctx *ctx, Field<PS, NC> &p, const Field<PS, NC> &r, int64_t V, cudaStream_t st) {
+void launch_p_update(lmb_ctx *ctx, const Field<PS, NC> &p, const Field<PS, NC> &pn, const Field<PS, NC> &r, int64_t V,
+                     cudaStream_t st) {
   if constexpr (PS != PREC_DOUBLE && NC == 12) {
     if (ctx->pair_sites && ctx->adj_sites && V % 2 == 0) {
-      cg_p_update_adj_kernel<PS><<<grid_for(V / 2, kBlasThreads), kBlasThreads, 0, st>>>(p, r, ctx->st_dev, V);
+      cg_p_update_adj_kernel<PS><<<grid_for(V / 2, kBlasThreads), kBlasThreads, 0, st>>>(p, pn, r, ctx->st_dev, V);
       return;
     }
   }
-  cg_p_update_kernel<PS, NC><<<grid_for(V, kBlasThreads), kBlasThreads, 0, st>>>(p, r, ctx->st_dev, V);
+  cg_p_update_kernel<PS, NC><<<grid_for(V, kBlasThreads), kBlasThreads, 0, st>>>(p, pn, r, ctx->st_dev, V);
 }
 
 // PS: precision of the iterated fields (DOUBLE = plain FP64 CG), PX: of x_low
@@ -329,23 +330,46 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
   int k1_n = 0, k2_n = 0;
 
   EpiStoreNorm<PS, NC> epi1{tl, ctx->st_dev, ctx->partials, ctx->counter};
-  EpiCGUpdate<PS, PX, NC> epi2{p, rl, xl, ctx->st_dev, ctx->partials, ctx->counter};
+  // x += alpha p waits until `depth` of them have come together (EpiCGUpdate).
+  // The direction of an iteration with n of them waiting is ring[n].  The extra
+  // directions take at most 4 GiB; where they do not fit x is updated more often.
+  Field<PS, NC> ring[kXDepth] = {p, p, p, p};
+  EpiCGUpdate<PS, PX, NC> epi2{{p, p, p, p}, rl, xl, ctx->st_dev, ctx->partials, ctx->counter};
+  int depth = 0;
+  auto make_ring = [&]() {
+    static const char *const name[kXDepth] = {"cg_p", "cg_p1", "cg_p2", "cg_p3"};
+    const int64_t want = std::min<int64_t>(kXDepth, 1 + ((int64_t)4 << 30) / (int64_t)Field<PS, NC>::bytes(V));
+    for (depth = 1; depth < want && make_field(ctx, name[depth], ring[depth], V); depth++) epi2.p[depth] = ring[depth];
+    if (depth < want) cudaGetLastError();  // the failed allocation's
+  };
+  auto flush_x = [&]() -> int {
+    if (!hs->npend) return LMB_OK;
+    cg_x_update_kernel<PS, PX, NC><<<bgrid, kBlasThreads, 0, st>>>(epi2, ctx->st_dev, hs->npend, V);
+    LMB_CHECK_LAUNCH(ctx);
+    nl++;
+    LMB_CUDA(ctx, cudaMemsetAsync(&ctx->st_dev->npend, 0, sizeof(int), st));
+    return LMB_OK;
+  };
   while (hs->status == ST_RUNNING) {
     const int it0 = hs->iter;
     const int small = prm->profile ? kNotSmall : op_cg_small(ctx, op, p, rl, tl, xl, st);
     if (small != kNotSmall && small != LMB_OK) return small;
     if (small == LMB_OK) nl++;
+    if (small == kNotSmall && !depth) make_ring();
     for (int i = 0; i < k && small == kNotSmall; i++) {
       if (prm->profile) cudaEventRecord(pool.ev[4 * i], st);
-      rc = op.template launch<PS, 0>(ctx, p, epi1, st);
+      const int cur = (hs->npend + i) % depth;
+      const bool last = cur == depth - 1;
+      rc = op.template launch<PS, 0>(ctx, ring[cur], epi1, st);
       if (rc) return rc;
       nl++;
       if (prm->profile) cudaEventRecord(pool.ev[4 * i + 1], st);
+      epi2.nx = last ? depth : 0;
       rc = op.template launch<PS, 1>(ctx, tl, epi2, st);
       if (rc) return rc;
       nl++;
       if (prm->profile) cudaEventRecord(pool.ev[4 * i + 2], st);
-      launch_p_update<PS, NC>(ctx, p, rl, V, st);
+      launch_p_update<PS, NC>(ctx, ring[cur], ring[last ? 0 : cur + 1], rl, V, st);
       LMB_CHECK_LAUNCH(ctx);
       nl++;
       if (prm->profile) cudaEventRecord(pool.ev[4 * i + 3], st);
@@ -368,13 +392,17 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
     }
     if (hs->status == ST_RELIABLE) {
       if constexpr (mixed) {
+        // the direction of the iteration that paused
+        const Field<PS, NC> &pc = ring[small == kNotSmall ? (hs->npend + depth - 1) % depth : 0];
+        rc = flush_x();
+        if (rc) return rc;
         fold_kernel<PX, NC><<<bgrid, kBlasThreads, 0, st>>>(x64, xl, V);
         LMB_CHECK_LAUNCH(ctx);
         nl++;
         // resume: the true-residual kernel runs regardless of the pause
         rc = true_residual(1);
         if (rc) return rc;
-        launch_p_update<PS, NC>(ctx, p, rl, V, st);
+        launch_p_update<PS, NC>(ctx, pc, p, rl, V, st);
         LMB_CHECK_LAUNCH(ctx);
         nl++;
         rc = read_state(ctx, st);
@@ -382,6 +410,8 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
       }
     }
   }
+  rc = flush_x();
+  if (rc) return rc;
   if constexpr (mixed) {
     fold_kernel<PX, NC><<<bgrid, kBlasThreads, 0, st>>>(x64, xl, V);
     LMB_CHECK_LAUNCH(ctx);

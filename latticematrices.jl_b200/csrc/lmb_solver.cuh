@@ -34,6 +34,8 @@ enum CGStatus {
   ST_BREAKDOWN = 5
 };
 
+constexpr int kXDepth = 4;  // most iterations whose updates of x are made together
+
 struct CGState {
   double rr;        // |r|^2 of the iterated residual
   double pAp, alpha, beta;
@@ -48,6 +50,8 @@ struct CGState {
   int maxiter;
   int status;
   int reliable_updates;
+  int npend;               // iterations whose x += alpha p is still to be added
+  double ahist[kXDepth];   // and their alpha
 };
 
 LMB_D void finalize_pAp(CGState *st, double pAp) {
@@ -205,37 +209,66 @@ struct EpiStoreNorm {  // K1
   }
 };
 
+// K2.  x enters no scalar of the iteration, so its updates are made for kXDepth
+// iterations at once, in their order (the same sum, rounding for rounding): x is
+// read and written a quarter as often, 288 of 2112 B per site and iteration of
+// the FP64 clover K2 and 144 of 640 B on int16 fields, and K3 writes the next
+// direction beside the ones that wait instead of over the last.  Bandwidth
+// bounds the FP64 K2, and it moves x's share no faster than the rest.  Solves,
+// updating x every 1, 2, 3, 4 iterations: clover FP64 24^3x48 226, 222, 219,
+// 218 ms, int16 32^3x64 283, 276, 274, 272, even/odd int16 24^3x48 34.6, 34.3,
+// 34.1, 34.1, HISQ FP32 32^3x64 185.6, 184.9, 184.2, 183.1, domain wall int16
+// 16^3x32x12 219, 216, 214, 214, Wilson FP64 16^3x32 15.0, 14.7, 14.5, 14.5.
+// (Loading x and p before r is stored, as an update in every iteration did,
+// spills 200 bytes here.)
 template <int PS, int PX, int NC = 12>
-struct EpiCGUpdate {  // K2
-  Field<PS, NC> p, r;
+struct EpiCGUpdate {
+  Field<PS, NC> p[kXDepth], r;
   Field<PX, NC> x;
   CGState *st;
   double *partials;
   unsigned *counter;
+  int nx = 1;               // p[0 .. nx-1] go into x; 0: in a later iteration
   double *local = nullptr;  // as EpiStoreNorm::local
   LMB_D bool skip() const { return ((volatile CGState *)st)->status != ST_RUNNING; }
-  LMB_D void finalize(double total) const { finalize_rr(st, total); }
-  template <typename R> LMB_D void operator()(int s, bool active, const Cx<R> *v) const {
-    double n2[1] = {0.0}, tot[1];
-    if (active) {
-      const R alpha = (R)st->alpha;
-      Cx<R> pv[NC], rv[NC], xv[NC];
-      p.load(s, pv);
-      r.load(s, rv);
-      x.load(s, xv);
+  LMB_D void finalize(double total) const {
+    if (nx) st->npend = 0;
+    else st->ahist[st->npend++] = st->alpha;
+    finalize_rr(st, total);
+  }
+  // x += sum_j alpha_j p[j] in the order of the iterations, the last of them
+  // this one's; x is read and written once for all of them
+  LMB_D double alpha_of(int j) const { return j == nx - 1 ? st->alpha : st->ahist[j]; }
+  template <typename R> LMB_D void add_x(int s) const {
+    Cx<R> xv[NC], pv[NC];
+    x.load(s, xv);
 #pragma unroll
-      for (int k = 0; k < NC; k++) {
-        rv[k] = rv[k] - alpha * v[k];
-        xv[k] = xv[k] + alpha * pv[k];
+    for (int j = 0; j < kXDepth; j++)
+      if (j < nx) {
+        const R a = (R)alpha_of(j);
+        p[j].load(s, pv);
+#pragma unroll
+        for (int k = 0; k < NC; k++) xv[k] = xv[k] + a * pv[k];
       }
-      r.store(s, rv);
-      x.store(s, xv);
-      n2[0] = sum_norm2(rv, NC);
-    }
-    if (grid_reduce<kDslashThreads, 1>(n2, partials, counter, tot) && threadIdx.x == 0) {
-      if (local) *local = tot[0];
-      else finalize_rr(st, tot[0]);
-    }
+    x.store(s, xv);
+  }
+  LMB_D void add_x_adj(int s0) const {
+    Cx2 xv[NC], pv[NC];
+    load_adj_rw(x, s0, xv);
+#pragma unroll
+    for (int j = 0; j < kXDepth; j++)
+      if (j < nx) {
+        const float2 pa = f2((float)alpha_of(j));
+        load_adj_rw(p[j], s0, pv);
+#pragma unroll
+        for (int k = 0; k < NC; k++) xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
+      }
+    store_adj(x, s0, xv);
+  }
+  template <typename R> LMB_D void operator()(int s, bool active, const Cx<R> *v) const {
+    double n2[1] = {0.0};
+    site_acc(s, active, v, n2);
+    finish(n2);
   }
   LMB_D void pair_adj(int s0, bool active, const Cx2 *v) const {
     double n2[1] = {0.0};
@@ -246,72 +279,68 @@ struct EpiCGUpdate {  // K2
   template <typename R> LMB_D void site_acc(int s, bool active, const Cx<R> *v, double (&red)[1]) const {
     if (active) {
       const R alpha = (R)st->alpha;
-      Cx<R> pv[NC], rv[NC], xv[NC];
-      p.load(s, pv);
+      Cx<R> rv[NC];
       r.load(s, rv);
-      x.load(s, xv);
 #pragma unroll
-      for (int k = 0; k < NC; k++) {
-        rv[k] = rv[k] - alpha * v[k];
-        xv[k] = xv[k] + alpha * pv[k];
-      }
+      for (int k = 0; k < NC; k++) rv[k] = rv[k] - alpha * v[k];
       r.store(s, rv);
-      x.store(s, xv);
       red[0] += sum_norm2(rv, NC);
+      if (nx) add_x<R>(s);
     }
   }
   // persistent kernels: update and add |r|^2 to red; finish() once per block
   LMB_D void pair_adj_acc(int s0, bool active, const Cx2 *v, double (&red)[1]) const {
     if (active) {
-      const float a = (float)st->alpha;
-      const float2 pa = f2(a), na = f2(-a);
-      Cx2 pv[NC], rv[NC], xv[NC];
-      load_adj_rw(p, s0, pv);
+      const float2 na = f2(-(float)st->alpha);
+      Cx2 rv[NC];
       load_adj_rw(r, s0, rv);
-      load_adj_rw(x, s0, xv);
       float2 q = f2(0.f);
 #pragma unroll
       for (int k = 0; k < NC; k++) {
         rv[k] = Cx2(fma2(na, v[k].re, rv[k].re), fma2(na, v[k].im, rv[k].im));
-        xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
         q = norm2_acc(rv[k], q);
       }
       store_adj(r, s0, rv);
-      store_adj(x, s0, xv);
       red[0] += (double)q.x + (double)q.y;
+      if (nx) add_x_adj(s0);
     }
   }
   LMB_D void finish(double (&red)[1]) const {
     double tot[1];
     if (grid_reduce<kDslashThreads, 1>(red, partials, counter, tot) && threadIdx.x == 0) {
       if (local) *local = tot[0];
-      else finalize_rr(st, tot[0]);
+      else finalize(tot[0]);
     }
   }
   LMB_D void pair(int s0, int s1, bool active, const Cx2 *v) const {
-    double n2[1] = {0.0}, tot[1];
+    double n2[1] = {0.0};
     if (active) {
-      const float a = (float)st->alpha;
-      const float2 pa = f2(a), na = f2(-a);
-      Cx2 pv[NC], rv[NC], xv[NC];
-      load2(p, s0, s1, pv);
+      const float2 na = f2(-(float)st->alpha);
+      Cx2 rv[NC];
       load2(r, s0, s1, rv);
-      load2(x, s0, s1, xv);
       float2 q = f2(0.f);
 #pragma unroll
       for (int k = 0; k < NC; k++) {
         rv[k] = Cx2(fma2(na, v[k].re, rv[k].re), fma2(na, v[k].im, rv[k].im));
-        xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
         q = norm2_acc(rv[k], q);
       }
       store2(r, s0, s1, rv);
-      store2(x, s0, s1, xv);
       n2[0] = (double)q.x + (double)q.y;
+      if (nx) {
+        Cx2 xv[NC], pv[NC];
+        load2(x, s0, s1, xv);
+#pragma unroll
+        for (int j = 0; j < kXDepth; j++)
+          if (j < nx) {
+            const float2 pa = f2((float)alpha_of(j));
+            load2(p[j], s0, s1, pv);
+#pragma unroll
+            for (int k = 0; k < NC; k++) xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
+          }
+        store2(x, s0, s1, xv);
+      }
     }
-    if (grid_reduce<kDslashThreads, 1>(n2, partials, counter, tot) && threadIdx.x == 0) {
-      if (local) *local = tot[0];
-      else finalize_rr(st, tot[0]);
-    }
+    finish(n2);
   }
 };
 
@@ -412,7 +441,7 @@ constexpr int kBlasThreads = 256;
 // K3: p = r + beta p
 template <int PS, int NC>
 __global__ void __launch_bounds__(kBlasThreads)
-    cg_p_update_kernel(Field<PS, NC> p, const Field<PS, NC> r, const CGState *st, int64_t V) {
+    cg_p_update_kernel(const Field<PS, NC> p, Field<PS, NC> pn, const Field<PS, NC> r, const CGState *st, int64_t V) {
   if (((volatile const CGState *)st)->status != ST_RUNNING) return;
   const int64_t s = (int64_t)blockIdx.x * kBlasThreads + threadIdx.x;
   if (s >= V) return;
@@ -423,14 +452,15 @@ __global__ void __launch_bounds__(kBlasThreads)
   r.load(s, rv);
 #pragma unroll
   for (int k = 0; k < NC; k++) pv[k] = rv[k] + beta * pv[k];
-  p.store(s, pv);
+  pn.store(s, pv);
 }
 
 // K3 on x-adjacent site pairs (V even; FP32 or int16 storage, NC = 12):
 // packed FP32 and 256-bit loads / stores, V/2 threads
 template <int PS>
 __global__ void __launch_bounds__(kBlasThreads)
-    cg_p_update_adj_kernel(Field<PS, 12> p, const Field<PS, 12> r, const CGState *st, int64_t V) {
+    cg_p_update_adj_kernel(const Field<PS, 12> p, Field<PS, 12> pn, const Field<PS, 12> r, const CGState *st,
+                           int64_t V) {
   if (((volatile const CGState *)st)->status != ST_RUNNING) return;
   const int64_t s = 2 * ((int64_t)blockIdx.x * kBlasThreads + threadIdx.x);
   if (s >= V) return;
@@ -440,7 +470,7 @@ __global__ void __launch_bounds__(kBlasThreads)
   load_adj_rw(r, s, rv);
 #pragma unroll
   for (int k = 0; k < 12; k++) pv[k] = Cx2(fma2(beta, pv[k].re, rv[k].re), fma2(beta, pv[k].im, rv[k].im));
-  store_adj(p, s, pv);
+  store_adj(pn, s, pv);
 }
 
 // dst = src (precision conversion)
@@ -460,6 +490,25 @@ __global__ void __launch_bounds__(kBlasThreads)
 }
 
 // x64 += x_low; x_low = 0
+// the iterations whose x += alpha p is still to be added (a solve that pauses
+// or ends between two updates of x)
+template <int PS, int PX, int NC>
+__global__ void __launch_bounds__(kBlasThreads)
+    cg_x_update_kernel(const EpiCGUpdate<PS, PX, NC> epi, const CGState *st, int n, int64_t V) {
+  const int64_t s = (int64_t)blockIdx.x * kBlasThreads + threadIdx.x;
+  if (s >= V) return;
+  typedef typename Real<PS>::type R;
+  Cx<R> xv[NC], pv[NC];
+  epi.x.load(s, xv);
+  for (int j = 0; j < n; j++) {
+    const R a = (R)st->ahist[j];
+    epi.p[j].load(s, pv);
+#pragma unroll
+    for (int k = 0; k < NC; k++) xv[k] = xv[k] + a * pv[k];
+  }
+  epi.x.store(s, xv);
+}
+
 template <int PX, int NC>
 __global__ void __launch_bounds__(kBlasThreads)
     fold_kernel(Field<PREC_DOUBLE, NC> x, Field<PX, NC> xl, int64_t V) {
