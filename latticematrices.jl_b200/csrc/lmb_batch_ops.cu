@@ -217,9 +217,9 @@ int batch_links_for(lmb_ctx *ctx, const lmb_batch_lattice &lat, const Geom &g, c
     ctx->batch_links.pop_back();
     return fail(ctx, LMB_ERR_UNSUPPORTED, "batched CG needs SU(3) links (deviation %.3g)", (double)dev);
   }
-  LMB_CUDA(ctx, cudaMalloc(&bl.d12, sizeof(double2) * 24 * V));
-  LMB_CUDA(ctx, cudaMalloc(&bl.f12, sizeof(float4) * 12 * V));
-  LMB_CUDA(ctx, cudaMalloc(&bl.h12, sizeof(int4) * 6 * V));
+  LMB_CUDA(ctx, device_malloc(ctx, &bl.d12, sizeof(double2) * 24 * V));
+  LMB_CUDA(ctx, device_malloc(ctx, &bl.f12, sizeof(float4) * 12 * V));
+  LMB_CUDA(ctx, device_malloc(ctx, &bl.h12, sizeof(int4) * 6 * V));
   links_to_recon12_kernel<<<grid_for(V, 256), 256, 0, st>>>(bl.d12, bl.f12, bl.h12, d, V);
   LMB_CHECK_LAUNCH(ctx);
   for (int mu = 0; mu < 4; mu++) {

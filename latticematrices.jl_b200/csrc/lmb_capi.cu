@@ -31,17 +31,17 @@ int ensure_link_precision(lmb_ctx *ctx, LinkSet &ls, int prec, cudaStream_t st, 
     float4 *f = nullptr;
     int4 *h = nullptr;
     if (prec == PREC_DOUBLE && ls.d12_version != ls.version) {
-      if (!ls.d12) LMB_CUDA(ctx, cudaMalloc(&ls.d12, sizeof(double2) * 24 * V));
+      if (!ls.d12) LMB_CUDA(ctx, device_malloc(ctx, &ls.d12, sizeof(double2) * 24 * V));
       d = ls.d12;
       ls.d12_version = ls.version;
     }
     if (prec == PREC_SINGLE && ls.f12_version != ls.version) {
-      if (!ls.f12) LMB_CUDA(ctx, cudaMalloc(&ls.f12, sizeof(float4) * 12 * V));
+      if (!ls.f12) LMB_CUDA(ctx, device_malloc(ctx, &ls.f12, sizeof(float4) * 12 * V));
       f = ls.f12;
       ls.f12_version = ls.version;
     }
     if (prec == PREC_HALF && ls.h12_version != ls.version) {
-      if (!ls.h12) LMB_CUDA(ctx, cudaMalloc(&ls.h12, sizeof(int4) * 6 * V));
+      if (!ls.h12) LMB_CUDA(ctx, device_malloc(ctx, &ls.h12, sizeof(int4) * 6 * V));
       h = ls.h12;
       ls.h12_version = ls.version;
     }
@@ -52,13 +52,13 @@ int ensure_link_precision(lmb_ctx *ctx, LinkSet &ls, int prec, cudaStream_t st, 
     return LMB_OK;
   }
   if (prec == PREC_SINGLE && ls.f_version != ls.version) {
-    if (!ls.f) LMB_CUDA(ctx, cudaMalloc(&ls.f, sizeof(float2) * n));
+    if (!ls.f) LMB_CUDA(ctx, device_malloc(ctx, &ls.f, sizeof(float2) * n));
     links_to_single_kernel<<<grid_for(V, 256), 256, 0, st>>>((float4 *)ls.f, ls.d, V);
     LMB_CHECK_LAUNCH(ctx);
     ls.f_version = ls.version;
   }
   if (prec == PREC_HALF && ls.h_version != ls.version) {
-    if (!ls.h) LMB_CUDA(ctx, cudaMalloc(&ls.h, sizeof(int) * n));
+    if (!ls.h) LMB_CUDA(ctx, device_malloc(ctx, &ls.h, sizeof(int) * n));
     links_to_half_kernel<<<grid_for(n, 256), 256, 0, st>>>(ls.h, ls.d, n, pow2_exponent(ls.scale));
     LMB_CHECK_LAUNCH(ctx);
     ls.h_version = ls.version;
@@ -129,7 +129,7 @@ int ensure_field_strength(lmb_ctx *ctx, cudaStream_t st) {
   const LinkSet &ls = ctx->links[LMB_LINKS_THIN];
   if (cc.F_valid && cc.F_links_version == ls.version) return LMB_OK;
   const int64_t V = ctx->g.V;
-  if (!cc.F) LMB_CUDA(ctx, cudaMalloc(&cc.F, sizeof(double2) * 54 * V));
+  if (!cc.F) LMB_CUDA(ctx, device_malloc(ctx, &cc.F, sizeof(double2) * 54 * V));
   if (ctx->dist && ctx->dist->split) {
     // a block of a process grid: the leaves reach the neighbours' links
     const int rc = dist_field_strength(ctx, st);
@@ -150,7 +150,7 @@ int ensure_clover(lmb_ctx *ctx, double coef, int prec, cudaStream_t st) {
   int rc = ensure_field_strength(ctx, st);
   if (rc) return rc;
   if (!cc.d_valid || cc.links_version != ls.version || cc.coef != coef) {
-    if (!cc.d) LMB_CUDA(ctx, cudaMalloc(&cc.d, sizeof(double2) * 36 * V));
+    if (!cc.d) LMB_CUDA(ctx, device_malloc(ctx, &cc.d, sizeof(double2) * 36 * V));
     clover_blocks_double_kernel<<<grid_for(V, 128), 128, 0, st>>>(cc.d, cc.F, ctx->g, coef);
     LMB_CHECK_LAUNCH(ctx);
     cc.d_valid = true;
@@ -166,14 +166,14 @@ int clover_convert(lmb_ctx *ctx, CloverCache &cc, int prec, cudaStream_t st) {
   const int64_t V = ctx->g.V;
   int rc = LMB_OK;
   if (prec == PREC_SINGLE && cc.f_version != cc.d_version) {
-    if (!cc.f) LMB_CUDA(ctx, cudaMalloc(&cc.f, sizeof(float4) * 18 * V));
+    if (!cc.f) LMB_CUDA(ctx, device_malloc(ctx, &cc.f, sizeof(float4) * 18 * V));
     clover_to_single_kernel<<<grid_for(V, 256), 256, 0, st>>>(cc.f, cc.d, V);
     LMB_CHECK_LAUNCH(ctx);
     cc.f_version = cc.d_version;
   }
   if (prec == PREC_HALF && cc.h_version != cc.d_version) {
-    if (!cc.h) LMB_CUDA(ctx, cudaMalloc(&cc.h, sizeof(int4) * 8 * V));
-    if (!cc.ht) LMB_CUDA(ctx, cudaMalloc(&cc.ht, sizeof(int2) * 2 * V));
+    if (!cc.h) LMB_CUDA(ctx, device_malloc(ctx, &cc.h, sizeof(int4) * 8 * V));
+    if (!cc.ht) LMB_CUDA(ctx, device_malloc(ctx, &cc.ht, sizeof(int2) * 2 * V));
     const float amax = device_absmax(ctx, cc.d, 36 * V, st, &rc);
     if (rc) return rc;
     const int kexp = pow2_exponent(amax);
@@ -286,6 +286,7 @@ lmb_ctx *lmb_create(int device) {
   if (const char *dw = getenv("LMB_DW_TWO_PASS")) ctx->dw_two_pass = atoi(dw) != 0;
   if (const char *pe = getenv("LMB_PERSISTENT")) ctx->persistent = atoi(pe) != 0;
   if (const char *bf = getenv("LMB_BATCH_FAMILY")) ctx->batch_family = atoi(bf);
+  if (const char *li = getenv("LMB_LIMITS")) ctx->limits = li;
   if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
     delete ctx;
     return nullptr;
@@ -393,7 +394,7 @@ int lmb_links_upload(lmb_ctx *ctx, int which, const void *const U[4], const uint
   if (same) return LMB_OK;
   cudaStream_t st = as_stream(stream);
   const int64_t V = ctx->g.V;
-  if (!ls.d) LMB_CUDA(ctx, cudaMalloc(&ls.d, sizeof(double2) * 36 * V));
+  if (!ls.d) LMB_CUDA(ctx, device_malloc(ctx, &ls.d, sizeof(double2) * 36 * V));
   if (ctx->dtype == LMB_DTYPE_C128)
     pack_links_kernel<double2><<<grid_for(V, 256), 256, 0, st>>>(
         ls.d, (const double2 *)U[0], (const double2 *)U[1], (const double2 *)U[2], (const double2 *)U[3], ctx->g,
@@ -637,7 +638,7 @@ int lmb_domainwall_set(lmb_ctx *ctx, int L5, double mass, double M, const double
     cudaFree(ctx->dw_coef);
     ctx->dw_coef = nullptr;
     ctx->dw_coef_cap = 0;
-    LMB_CUDA(ctx, cudaMalloc(&ctx->dw_coef, sizeof(double) * 3 * L5));
+    LMB_CUDA(ctx, device_malloc(ctx, &ctx->dw_coef, sizeof(double) * 3 * L5));
     ctx->dw_coef_cap = 3 * L5;
   }
   // ordered on the stream after the kernels that read the previous values

@@ -4,9 +4,12 @@
 #include <cuda_runtime.h>
 
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
+#include <cstdlib>
 #include <deque>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -130,6 +133,13 @@ struct lmb_ctx {
   };
   std::map<std::string, EoTag> eo_tags;
   std::map<std::string, std::pair<void *, size_t>> buffers;
+  // workspaces the library can do without (spare_workspace): freed when a
+  // needed allocation is refused, unless a running solve holds them
+  std::set<std::string> spare;
+  int spare_held = 0;
+  // bounds the environment may lower (LMB_LIMITS="key=value,..", read by
+  // lmb_create; limit_of), so that the ways round a refusal can be taken
+  std::string limits;
   double *partials = nullptr;
   size_t partials_cap = 0;
   unsigned *counter = nullptr;
@@ -167,17 +177,101 @@ inline int fail(lmb_ctx *ctx, int code, const char *fmt, ...) {
                          __FILE__, __LINE__);                                             \
   } while (0)
 
+// `most`, or the lower bound set for `key`
+inline int64_t limit_of(const lmb_ctx *ctx, const std::string &key, int64_t most) {
+  const size_t at = ("," + ctx->limits).find("," + key + "=");
+  if (at == std::string::npos) return most;
+  const int64_t v = atoll(ctx->limits.c_str() + at + key.size() + 1);
+  return v < most ? v : most;
+}
+
+// whether `bytes` more keep the workspaces within the bound set for them
+inline bool workspace_fits(const lmb_ctx *ctx, size_t bytes) {
+  if (ctx->limits.empty()) return true;
+  int64_t used = (int64_t)bytes;
+  for (auto &kv : ctx->buffers) used += (int64_t)kv.second.second;
+  return used <= limit_of(ctx, "workspace", INT64_MAX);
+}
+inline void drop_workspace(lmb_ctx *ctx, const std::string &name) {
+  auto it = ctx->buffers.find(name);
+  if (it == ctx->buffers.end()) return;
+  cudaFree(it->second.first);
+  ctx->buffers.erase(it);
+}
+// frees the spare workspaces; false: there are none, or they are in use
+inline bool release_spare(lmb_ctx *ctx) {
+  if (ctx->spare_held || ctx->spare.empty()) return false;
+  for (auto &name : ctx->spare) drop_workspace(ctx, name);
+  ctx->spare.clear();
+  return true;
+}
+
+// keeps the spare workspaces from take() to the end of its scope
+struct SpareHold {
+  lmb_ctx *ctx;
+  bool held = false;
+  explicit SpareHold(lmb_ctx *c) : ctx(c) {}
+  SpareHold(const SpareHold &) = delete;
+  void take() {
+    if (!held) ctx->spare_held++;
+    held = true;
+  }
+  ~SpareHold() {
+    if (held) ctx->spare_held--;
+  }
+};
+
+// cudaMalloc that gives up the spare workspaces where it is refused, and
+// leaves no error behind for the next launch check
+inline cudaError_t device_malloc(lmb_ctx *ctx, void **p, size_t bytes) {
+  cudaError_t e;
+  while ((e = cudaMalloc(p, bytes)) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    if (!release_spare(ctx)) break;
+  }
+  return e;
+}
+template <typename T>
+cudaError_t device_malloc(lmb_ctx *ctx, T **p, size_t bytes) {
+  void *q = nullptr;
+  const cudaError_t e = device_malloc(ctx, &q, bytes);
+  *p = (T *)q;
+  return e;
+}
+
 // named workspace, grown on demand (never shrinks until lmb_destroy)
 inline void *workspace(lmb_ctx *ctx, const std::string &name, size_t bytes) {
   auto it = ctx->buffers.find(name);
   if (it != ctx->buffers.end() && it->second.second >= bytes) return it->second.first;
-  if (it != ctx->buffers.end()) {
-    cudaFree(it->second.first);
-    ctx->buffers.erase(it);
-  }
+  drop_workspace(ctx, name);
+  ctx->spare.erase(name);
+  while (!workspace_fits(ctx, bytes))
+    if (!release_spare(ctx)) return nullptr;
   void *p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
+  if (device_malloc(ctx, &p, bytes) != cudaSuccess) return nullptr;
   ctx->buffers[name] = {p, bytes};
+  return p;
+}
+
+// named workspace that only makes a call faster: nullptr unless an eighth of
+// the device stays free beside it for what the caller, other contexts and
+// libraries allocate later
+inline void *spare_workspace(lmb_ctx *ctx, const std::string &name, size_t bytes) {
+  auto it = ctx->buffers.find(name);
+  if (it != ctx->buffers.end() && it->second.second >= bytes) return it->second.first;
+  drop_workspace(ctx, name);
+  ctx->spare.erase(name);
+  size_t avail = 0, total = 0;
+  if (!workspace_fits(ctx, bytes) || cudaMemGetInfo(&avail, &total) != cudaSuccess || avail < bytes + total / 8)
+    return nullptr;
+  void *p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  ctx->buffers[name] = {p, bytes};
+  ctx->spare.insert(name);
   return p;
 }
 
@@ -187,18 +281,18 @@ inline bool ensure_partials(lmb_ctx *ctx, size_t blocks, int nval) {
   if (ctx->partials) cudaFree(ctx->partials);
   ctx->partials = nullptr;
   ctx->partials_cap = 0;
-  if (cudaMalloc(&ctx->partials, need * sizeof(double)) != cudaSuccess) return false;
+  if (device_malloc(ctx, &ctx->partials, need * sizeof(double)) != cudaSuccess) return false;
   ctx->partials_cap = need;
   return true;
 }
 
 // a field of V sites (default: the context's 4D volume)
 template <int P, int NC>
-inline bool make_field(lmb_ctx *ctx, const std::string &name, Field<P, NC> &f, int64_t V = -1) {
+inline bool make_field(lmb_ctx *ctx, const std::string &name, Field<P, NC> &f, int64_t V = -1, bool spare = false) {
   if (V < 0) V = ctx->g.V;
   f.V = V;
   const size_t nb = Field<P, NC>::bytes(V), mb = Field<P, NC>::norm_bytes(V);
-  void *p = workspace(ctx, name, nb + mb + 256);
+  void *p = (spare ? spare_workspace : workspace)(ctx, name, nb + mb + 256);
   if (!p) return false;
   f.data = (decltype(f.data))p;
   f.norm = mb ? (float *)((char *)p + ((nb + 255) / 256) * 256) : nullptr;

@@ -106,7 +106,7 @@ int dist_boundary(lmb_ctx *ctx, int depth, bool pairs, const int **list, int *n)
     }
     int *dev = nullptr;
     if (!sites.empty()) {
-      LMB_CUDA(ctx, cudaMalloc(&dev, sizeof(int) * sites.size()));
+      LMB_CUDA(ctx, device_malloc(ctx, &dev, sizeof(int) * sites.size()));
       LMB_CUDA(ctx, cudaMemcpy(dev, sites.data(), sizeof(int) * sites.size(), cudaMemcpyHostToDevice));
     }
     it = d->boundary.emplace(key, std::make_pair(dev, (int)sites.size())).first;
@@ -139,7 +139,7 @@ int dist_link_ghosts(lmb_ctx *ctx, int which, int depth, int prec, bool allow_re
       gs.version = version;
       if (!((d->split >> mu) & 1)) continue;
       const int64_t Vg = (int64_t)depth * dv.face[mu];
-      LMB_CUDA(ctx, cudaMalloc(&gs.d, sizeof(double2) * 36 * Vg));
+      LMB_CUDA(ctx, device_malloc(ctx, &gs.d, sizeof(double2) * 36 * Vg));
       LMB_CUDA(ctx, cudaMemsetAsync(gs.d, 0, sizeof(double2) * 36 * Vg, st));
       const unsigned grid = grid_for(Vg, 256);
       if (ctx->dtype == LMB_DTYPE_C128)

@@ -26,6 +26,10 @@ int op_unpack_out(lmb_ctx *ctx, const Op &, void *dst, const Field<PS, NC> &f, c
   return unpack_out(ctx, dst, f, st);
 }
 
+// the workspaces a precision's launches of the operator take inside a solve
+// (made before the solve spends memory it could do without)
+template <int PS, class Op> bool op_reserve(lmb_ctx *, const Op &) { return true; }
+
 // all iterations up to the next status change in one launch (lmb_small.cuh):
 // LMB_OK or an error; kNotSmall where the operator or the lattice has no such
 // kernel
@@ -332,15 +336,22 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
   EpiStoreNorm<PS, NC> epi1{tl, ctx->st_dev, ctx->partials, ctx->counter};
   // x += alpha p waits until `depth` of them have come together (EpiCGUpdate).
   // The direction of an iteration with n of them waiting is ring[n].  The extra
-  // directions take at most 4 GiB; where they do not fit x is updated more often.
+  // directions take at most 4 GiB of memory that nothing else of the solve asks
+  // for; where there is none x is updated more often, and a later call that
+  // runs out of memory takes them back (release_spare).
   Field<PS, NC> ring[kXDepth] = {p, p, p, p};
   EpiCGUpdate<PS, PX, NC> epi2{{p, p, p, p}, rl, xl, ctx->st_dev, ctx->partials, ctx->counter};
   int depth = 0;
-  auto make_ring = [&]() {
+  SpareHold hold(ctx);
+  auto make_ring = [&]() -> bool {
     static const char *const name[kXDepth] = {"cg_p", "cg_p1", "cg_p2", "cg_p3"};
-    const int64_t want = std::min<int64_t>(kXDepth, 1 + ((int64_t)4 << 30) / (int64_t)Field<PS, NC>::bytes(V));
-    for (depth = 1; depth < want && make_field(ctx, name[depth], ring[depth], V); depth++) epi2.p[depth] = ring[depth];
-    if (depth < want) cudaGetLastError();  // the failed allocation's
+    if (!op_reserve<PS>(ctx, op) || !op_reserve<PREC_DOUBLE>(ctx, op)) return false;
+    const int64_t want =
+        std::min(limit_of(ctx, "directions", kXDepth), 1 + ((int64_t)4 << 30) / (int64_t)Field<PS, NC>::bytes(V));
+    for (depth = 1; depth < want && make_field(ctx, name[depth], ring[depth], V, true); depth++)
+      epi2.p[depth] = ring[depth];
+    if (depth > 1) hold.take();
+    return true;
   };
   auto flush_x = [&]() -> int {
     if (!hs->npend) return LMB_OK;
@@ -355,7 +366,8 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
     const int small = prm->profile ? kNotSmall : op_cg_small(ctx, op, p, rl, tl, xl, st);
     if (small != kNotSmall && small != LMB_OK) return small;
     if (small == LMB_OK) nl++;
-    if (small == kNotSmall && !depth) make_ring();
+    if (small == kNotSmall && !depth && !make_ring())
+      return fail(ctx, LMB_ERR_CUDA, "out of device memory (CG operator workspaces)");
     for (int i = 0; i < k && small == kNotSmall; i++) {
       if (prm->profile) cudaEventRecord(pool.ev[4 * i], st);
       const int cur = (hs->npend + i) % depth;

@@ -131,7 +131,7 @@ int naik_planes(lmb_ctx *ctx, const double2 *W, double2 *L, cudaStream_t st) {
 double2 *derived_planes(lmb_ctx *ctx, int which) {
   LinkSet &ls = ctx->links[which];
   ls.valid = false;
-  if (!ls.d && cudaMalloc(&ls.d, sizeof(double2) * 36 * ctx->g.V) != cudaSuccess) ls.d = nullptr;
+  if (!ls.d && device_malloc(ctx, &ls.d, sizeof(double2) * 36 * ctx->g.V) != cudaSuccess) ls.d = nullptr;
   return ls.d;
 }
 int install_links(lmb_ctx *ctx, int which, cudaStream_t st) {

@@ -30,6 +30,11 @@ struct DWPolicy {
     return one_pass(ctx) && ctx->pair_sites && ctx->adj_sites && ctx->dw_L5 % 2 == 0 &&
            fills_device(ctx, ctx->g.V * (ctx->dw_L5 / 2), P == PREC_HALF ? 2 : 3, 4);
   }
+  // the field between two passes (the two-pass launches, the small-lattice D5^+)
+  template <int P> static bool make_tmp(lmb_ctx *ctx, Field<P, 12> &f) {
+    return make_field(ctx, P == PREC_DOUBLE ? "dw_tmp_d" : (P == PREC_SINGLE ? "dw_tmp_s" : "dw_tmp_h"), f,
+                      ctx->g.V * ctx->dw_L5);
+  }
   // blocks of the largest launch (the one-pass adjoint holds whole 4D points)
   static int64_t max_blocks(const lmb_ctx *ctx) {
     const int64_t flat = grid_for(ctx->g.V * ctx->dw_L5, kDslashThreads);
@@ -45,9 +50,6 @@ struct DWPolicy {
   int launch_g(lmb_ctx *ctx, const Field<P, 12> &in, const G &U, const Epi &epi, cudaStream_t st) const {
     typedef typename Real<P>::type R;
     const int64_t V4 = ctx->g.V, V5 = V4 * ctx->dw_L5;
-    Field<P, 12> tmp;
-    if (!make_field(ctx, P == PREC_DOUBLE ? "dw_tmp_d" : (P == PREC_SINGLE ? "dw_tmp_s" : "dw_tmp_h"), tmp, V5))
-      return fail(ctx, LMB_ERR_CUDA, "out of device memory (domain-wall workspace)");
     const DWParams d = params(ctx);
     const unsigned grid = grid_for(V5, kDslashThreads);
     if constexpr (P != PREC_DOUBLE) {
@@ -73,6 +75,8 @@ struct DWPolicy {
       LMB_CHECK_LAUNCH(ctx);
       return LMB_OK;
     }
+    Field<P, 12> tmp;
+    if (!make_tmp(ctx, tmp)) return fail(ctx, LMB_ERR_CUDA, "out of device memory (domain-wall workspace)");
     if constexpr (!DAG) {
       dw_fifth_kernel<P><<<grid, kDslashThreads, 0, st>>>(tmp, in, V4, d, epi);
       dw_stencil_kernel<R, 0, 1><<<grid, kDslashThreads, 0, st>>>(ctx->g, tmp, in, U, d, epi);
@@ -98,6 +102,10 @@ inline int64_t op_volume(const lmb_ctx *ctx, const DWPolicy &) { return ctx->g.V
 template <> struct DirectOut<DWPolicy> { static constexpr bool value = true; };
 inline int op_slices(const lmb_ctx *ctx, const DWPolicy &) { return ctx->dw_L5; }
 inline int64_t op_max_blocks(const lmb_ctx *ctx, const DWPolicy &) { return DWPolicy::max_blocks(ctx); }
+template <int PS> bool op_reserve(lmb_ctx *ctx, const DWPolicy &) {
+  Field<PS, 12> f;
+  return DWPolicy::one_pass(ctx) || DWPolicy::make_tmp(ctx, f);
+}
 template <int PS, int NC>
 int op_pack_in(lmb_ctx *ctx, const DWPolicy &, Field<PS, NC> &f, const void *src, cudaStream_t st) {
   const unsigned grid = grid_for(ctx->g.V * ctx->dw_L5, 256);

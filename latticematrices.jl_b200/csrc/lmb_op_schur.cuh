@@ -76,6 +76,10 @@ struct SchurPolicy {
     }
     return ensure_eo_copies(ctx, prec, clover, st);
   }
+  // the odd half field between the two hops
+  template <int P> static bool make_tmp(lmb_ctx *ctx, Field<P, 12> &t) {
+    return make_field(ctx, P == PREC_DOUBLE ? "eo_t_d" : (P == PREC_SINGLE ? "eo_t_s" : "eo_t_h"), t, ctx->g.V / 2);
+  }
   template <int P, bool CL, int DAG, class G, class Epi>
   void launch_cl(lmb_ctx *ctx, const Field<P, 12> &in, const Field<P, 12> &t, const G &U, const Epi &epi,
                  cudaStream_t st) const {
@@ -105,8 +109,7 @@ struct SchurPolicy {
   template <int P, int DAG, class G, class Epi>
   int launch_g(lmb_ctx *ctx, const Field<P, 12> &in, const G &U, const Epi &epi, cudaStream_t st) const {
     Field<P, 12> t;
-    if (!make_field(ctx, P == PREC_DOUBLE ? "eo_t_d" : (P == PREC_SINGLE ? "eo_t_s" : "eo_t_h"), t, ctx->g.V / 2))
-      return fail(ctx, LMB_ERR_CUDA, "out of device memory (even/odd workspace)");
+    if (!make_tmp(ctx, t)) return fail(ctx, LMB_ERR_CUDA, "out of device memory (even/odd workspace)");
     if (clover) launch_cl<P, true, 1 - DAG>(ctx, in, t, U, epi, st);
     else launch_cl<P, false, 1 - DAG>(ctx, in, t, U, epi, st);
     LMB_CHECK_LAUNCH(ctx);
@@ -124,6 +127,10 @@ struct SchurPolicy {
 // the CG driver's b and x of the Schur system are FP64 half fields of the
 // even/odd solve (passed as Field pointers), not padded reference arrays
 inline int64_t op_volume(const lmb_ctx *ctx, const SchurPolicy &) { return ctx->g.V / 2; }
+template <int PS> bool op_reserve(lmb_ctx *ctx, const SchurPolicy &) {
+  Field<PS, 12> t;
+  return SchurPolicy::make_tmp(ctx, t);
+}
 template <int PS, int NC>
 int op_pack_in(lmb_ctx *ctx, const SchurPolicy &, Field<PS, NC> &f, const void *src, cudaStream_t st) {
   const Field<PREC_DOUBLE, NC> &h = *(const Field<PREC_DOUBLE, NC> *)src;

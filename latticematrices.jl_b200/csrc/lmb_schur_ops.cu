@@ -14,7 +14,7 @@ int ensure_clover_inverse(lmb_ctx *ctx, int prec, cudaStream_t st) {
   const int64_t V = ctx->g.V;
   if (!cc.d_valid) return fail(ctx, LMB_ERR_STATE, "clover blocks have not been built");
   if (!ci.d_valid || ci.src_version != cc.d_version) {
-    if (!ci.d) LMB_CUDA(ctx, cudaMalloc(&ci.d, sizeof(double2) * 36 * V));
+    if (!ci.d) LMB_CUDA(ctx, device_malloc(ctx, &ci.d, sizeof(double2) * 36 * V));
     unsigned *bad = (unsigned *)workspace(ctx, "clover_inv_bad", sizeof(unsigned));
     if (!bad) return fail(ctx, LMB_ERR_CUDA, "out of device memory (clover inverse)");
     LMB_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(unsigned), st));

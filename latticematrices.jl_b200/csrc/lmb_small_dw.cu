@@ -113,10 +113,9 @@ struct SmallDW {
 template <int PS, int PX>
 int op_cg_small(lmb_ctx *ctx, const DWPolicy &op, const Field<PS, 12> &p, const Field<PS, 12> &r,
                 const Field<PS, 12> &t, const Field<PX, 12> &x, cudaStream_t st) {
-  const int64_t V5 = ctx->g.V * ctx->dw_L5;
   if (!ctx->persistent) return kNotSmall;
   Field<PS, 12> mid;
-  if (!make_field(ctx, PS == PREC_DOUBLE ? "dw_tmp_d" : (PS == PREC_SINGLE ? "dw_tmp_s" : "dw_tmp_h"), mid, V5))
+  if (!DWPolicy::make_tmp(ctx, mid))
     return fail(ctx, LMB_ERR_CUDA, "out of device memory (domain-wall workspace)");
   const DWParams d = op.params(ctx);
   const LinkSet &ls = ctx->links[LMB_LINKS_THIN];

@@ -1,0 +1,147 @@
+"""GPU: the ways round a refused allocation or launch, taken under bounds that
+LMB_LIMITS sets (lmb_create reads it), and the results on them.
+
+A bound on the workspaces refuses on the host what the device would refuse when
+it is full; nothing here fills the device."""
+import numpy as np
+import pytest
+
+import refdata as rd
+
+pytestmark = pytest.mark.gpu
+PHASES = (1, 1, 1, -1)
+
+
+@pytest.fixture(scope="module")
+def lmb():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import lmb200
+    lmb200.load()
+    return lmb200
+
+
+def _links(lmb, U, nw):
+    return [lmb.LatticeMatrix.from_array(u, nw=nw) for u in U]
+
+
+def _field(lmb, orc, L, spins, seed, nw):
+    return lmb.LatticeMatrix.from_array(orc.gaussian_field(L, 3, spins, seed), nw=nw, phases=PHASES)
+
+
+def _clover_solve(lmb, orc, precision, **kw):
+    L = (6, 4, 4, 8)
+    D = lmb.WilsonDiracCloverOperator4D(_links(lmb, orc.random_su3_links(L, 0.25, 11), 1), 0.12, 1.0)
+    b = _field(lmb, orc, L, 4, 12, 1)
+    x = b.similar()
+    return lmb.cg_(x, lmb.DdagDOp(D, b.similar()), b, precision=precision, **kw), [x.gather_matrix()]
+
+
+def _staggered_solve(lmb, orc, precision, **kw):
+    L = (6, 4, 4, 8)
+    D = lmb.StaggeredDiracOperator4D(_links(lmb, orc.random_su3_links(L, 0.25, 13), 3), 0.3)
+    b = _field(lmb, orc, L, 1, 14, 3)
+    x = b.similar()
+    return lmb.cg_(x, lmb.DdagDOp(D, b.similar()), b, precision=precision, **kw), [x.gather_matrix()]
+
+
+def _evenodd_solve(lmb, orc, precision, **kw):
+    L = (4, 4, 4, 6)
+    D = lmb.WilsonDiracCloverOperator4D(_links(lmb, orc.random_su3_links(L, 0.25, 15), 1), 0.12, 1.0)
+    b = _field(lmb, orc, L, 4, 16, 1)
+    x = b.similar()
+    return lmb.solve_evenodd_(x, D, b, precision=precision, **kw), [x.gather_matrix()]
+
+
+def _domainwall_solve(lmb, orc, precision, **kw):
+    L, L5 = (4, 4, 4, 4), 6
+    D = lmb.D5DW_MobiusDomainwallOperator5D(_links(lmb, orc.random_su3_links(L, 0.25, 17), 1), L5, 0.2, -1.4, 1.5, 0.5)
+    flat = orc.gaussian_field(L[:3] + (L[3] * L5,), 3, 4, 18)
+    b = lmb.LatticeMatrix.from_array(np.asfortranarray(flat.reshape((3, 4) + L + (L5,), order="F")), 5, nw=1,
+                                     phases=PHASES + (1,))
+    x = b.similar()
+    return lmb.cg_(x, lmb.DdagDOp(D, b.similar()), b, precision=precision, **kw), [x.gather_matrix()]
+
+
+def _hisq_force(lmb, orc, precision, **kw):
+    L = (4, 4, 4, 4)
+    U = _links(lmb, orc.random_su3_links(L, 0.2, 19), 3)
+    dU = [u.similar() for u in U]
+    res = lmb.hisq_fermion_force_(dU, lmb.HISQDiracCache4D(U, 0.3), _field(lmb, orc, L, 1, 20, 3), precision=precision,
+                                  **kw)
+    return res, [d.gather_matrix() for d in dU]
+
+
+def _clover_force(lmb, orc, precision, **kw):
+    L = (4, 4, 4, 4)
+    U = _links(lmb, orc.random_su3_links(L, 0.2, 21), 1)
+    dU = [u.similar() for u in U]
+    res = lmb.wilson_clover_fermion_force_(dU, lmb.WilsonDiracCloverOperator4D(U, 0.12, 1.0),
+                                           _field(lmb, orc, L, 4, 22, 1), precision=precision, **kw)
+    return res, [d.gather_matrix() for d in dU]
+
+
+def _least(fits):
+    """The smallest number of bytes, to 4 KiB, for which fits(bytes) holds."""
+    lo, hi = 0, 1 << 16
+    while not fits(hi):
+        lo, hi = hi, 2 * hi
+        assert hi < 1 << 34
+    while hi - lo > 4096:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if fits(mid) else (mid, hi)
+    return hi
+
+
+def _fits(lmb, call):
+    try:
+        call()
+    except lmb.LMBError as e:
+        assert "out of device memory" in str(e)
+        return False
+    return True
+
+
+# Every number of directions, and every number of updates of x that still wait
+# when the solve pauses or stops: the same sum in the same order.  A solve that
+# stops with some of them waiting launches one kernel more, which shows how many
+# directions it ran with.
+@pytest.mark.parametrize("solve", [_clover_solve, _staggered_solve])
+@pytest.mark.parametrize("precision", ["double", "single", "half"])
+def test_solution_does_not_depend_on_the_directions(lmb, orc, monkeypatch, solve, precision):
+    monkeypatch.setenv("LMB_PERSISTENT", "0")
+    for maxiter in (2, 3, 4, 300):
+        out = []
+        for n in (1, 2, 3, 4):
+            monkeypatch.setenv("LMB_LIMITS", f"directions={n}")
+            out.append(solve(lmb, orc, precision, rtol=1e-9 if maxiter == 300 else 1e-14, maxiter=maxiter))
+        assert out[0][0].converged == (maxiter == 300)
+        for res, (x,) in out[1:]:
+            assert (res.iterations, res.reason) == (out[0][0].iterations, out[0][0].reason)
+            np.testing.assert_array_equal(x, out[0][1][0])
+        if precision == "double" and maxiter < 300:
+            more = [res.kernel_launches - out[0][0].kernel_launches for res, _ in out]
+            assert more == [1 if maxiter % n else 0 for n in (1, 2, 3, 4)]
+
+
+# The extra directions are no reason for a call to run out of memory: neither
+# what the solve itself asks for after them (the workspaces of its FP64 updates)
+# nor what follows on the same context (the gradient of a force, the residual of
+# an even/odd solve) is refused because of them.
+@pytest.mark.parametrize("call", [_domainwall_solve, _evenodd_solve, _hisq_force, _clover_force])
+@pytest.mark.parametrize("precision", ["double", "half"])
+def test_directions_take_no_memory_that_is_needed(lmb, orc, monkeypatch, call, precision):
+    monkeypatch.setenv("LMB_PERSISTENT", "0")
+    monkeypatch.setenv("LMB_DW_TWO_PASS", "1")
+
+    def run(limits):
+        monkeypatch.setenv("LMB_LIMITS", limits)
+        return call(lmb, orc, precision, rtol=1e-9)
+    least = _least(lambda n: _fits(lmb, lambda: run(f"directions=1,workspace={n}")))
+    (one, want), (res, got) = run(f"directions=1,workspace={least}"), run(f"workspace={least}")
+    assert one.converged and res.converged and res.iterations == one.iterations
+    for g, w in zip(got, want):
+        assert rd.rel_err(g, w) <= 1e-12
+    monkeypatch.setenv("LMB_LIMITS", "workspace=4096")
+    assert not _fits(lmb, lambda: call(lmb, orc, precision))
