@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -137,6 +138,7 @@ struct lmb_ctx {
   // needed allocation is refused, unless a running solve holds them
   std::set<std::string> spare;
   int spare_held = 0;
+  int growths = 0;  // workspaces replaced by larger ones so far
   // bounds the environment may lower (LMB_LIMITS="key=value,..", read by
   // lmb_create; limit_of), so that the ways round a refusal can be taken
   std::string limits;
@@ -192,11 +194,12 @@ inline bool workspace_fits(const lmb_ctx *ctx, size_t bytes) {
   for (auto &kv : ctx->buffers) used += (int64_t)kv.second.second;
   return used <= limit_of(ctx, "workspace", INT64_MAX);
 }
-inline void drop_workspace(lmb_ctx *ctx, const std::string &name) {
+inline bool drop_workspace(lmb_ctx *ctx, const std::string &name) {
   auto it = ctx->buffers.find(name);
-  if (it == ctx->buffers.end()) return;
+  if (it == ctx->buffers.end()) return false;
   cudaFree(it->second.first);
   ctx->buffers.erase(it);
+  return true;
 }
 // frees the spare workspaces; false: there are none, or they are in use
 inline bool release_spare(lmb_ctx *ctx) {
@@ -240,11 +243,13 @@ cudaError_t device_malloc(lmb_ctx *ctx, T **p, size_t bytes) {
   return e;
 }
 
-// named workspace, grown on demand (never shrinks until lmb_destroy)
+// Named workspace, grown on demand (never shrinks until lmb_destroy).  Growing
+// frees the old one, which waits for the device: a call that takes one name at
+// several sizes asks for the largest first.
 inline void *workspace(lmb_ctx *ctx, const std::string &name, size_t bytes) {
   auto it = ctx->buffers.find(name);
   if (it != ctx->buffers.end() && it->second.second >= bytes) return it->second.first;
-  drop_workspace(ctx, name);
+  if (drop_workspace(ctx, name) && ctx->growths++ >= limit_of(ctx, "growths", INT_MAX)) return nullptr;
   ctx->spare.erase(name);
   while (!workspace_fits(ctx, bytes))
     if (!release_spare(ctx)) return nullptr;

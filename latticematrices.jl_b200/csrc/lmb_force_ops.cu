@@ -53,6 +53,20 @@ struct Fat7Launch {
 Fat7Launch fat7_launch(const Geom &g, int fields) {
   return Fat7Launch{g.V <= (1 << 16) ? 4 : 1, (int64_t)fields * 9 * g.V};
 }
+// fields of nine planes per direction: S and M (M+ and M- with the Lepage
+// term) of the three axes, for the gradient twice
+int fat7_fields(bool lepage, bool gradient) { return (lepage ? 9 : 6) * (gradient ? 2 : 1); }
+double2 *fat7_workspace(lmb_ctx *ctx, const Fat7Launch &l) {
+  return (double2 *)workspace(ctx, "fat7", sizeof(double2) * l.nmu * l.per_mu);
+}
+// A chain's largest stage is its second level's, with the Lepage term; asked
+// for first, so that the first level's is not freed for it (first smearing and
+// link gradient of a new operator: see hisq_links_from_thin and
+// hisq_pullback_planes)
+int fat7_reserve(lmb_ctx *ctx, bool gradient) {
+  if (fat7_workspace(ctx, fat7_launch(ctx->g, fat7_fields(true, gradient)))) return LMB_OK;
+  return fail(ctx, LMB_ERR_CUDA, "out of device memory (Fat7 stages)");
+}
 
 // block shapes of a stage for the directions mu0 .. mu0 + nmu - 1, and the
 // largest number of blocks
@@ -98,9 +112,8 @@ void fat7_sum(lmb_ctx *ctx, const Fat7Launch &l, const double2 *U, double2 *out,
 int fat7_planes(lmb_ctx *ctx, const double2 *U, double2 *V, const double *coef, cudaStream_t st) {
   const int64_t F3 = 27 * ctx->g.V;  // the three axes' fields
   const bool lepage = coef[4] != 0.0;
-  const int fields = lepage ? 9 : 6;
-  const Fat7Launch l = fat7_launch(ctx->g, fields);
-  double2 *work = (double2 *)workspace(ctx, "fat7", sizeof(double2) * l.nmu * l.per_mu);
+  const Fat7Launch l = fat7_launch(ctx->g, fat7_fields(lepage, false));
+  double2 *work = fat7_workspace(ctx, l);
   if (!work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing staples)");
   const Fat7Field f{U, work, work + F3, lepage ? work + 2 * F3 : work + F3, coef[1]};
   for (int mu = 0; mu < 4; mu += l.nmu) {
@@ -155,9 +168,8 @@ int fat7_pullback_planes(lmb_ctx *ctx, const double2 *U, const double2 *dV, doub
                          cudaStream_t st) {
   const int64_t F3 = 27 * ctx->g.V;
   const bool lepage = coef[4] != 0.0;
-  const int fields = lepage ? 18 : 12;
-  const Fat7Launch l = fat7_launch(ctx->g, fields);
-  double2 *work = (double2 *)workspace(ctx, "fat7", sizeof(double2) * l.nmu * l.per_mu);
+  const Fat7Launch l = fat7_launch(ctx->g, fat7_fields(lepage, true));
+  double2 *work = fat7_workspace(ctx, l);
   if (!work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (force staples)");
   const Fat7Field fu{U, work, work + F3, lepage ? work + 4 * F3 : work + F3, 0.0};
   const Fat7Field fg{dV, work + 2 * F3, work + 3 * F3, lepage ? work + 5 * F3 : work + 3 * F3, coef[1]};
@@ -188,6 +200,7 @@ int hisq_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_DOU
   const double c_level1[5] = {1.0 / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, 0.0};
   const double c_level2[5] = {1.0 + naik_epsilon / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, -1.0 / 8};
   int rc;
+  if ((rc = fat7_reserve(ctx, true))) return rc;
   // recompute the smearing levels the pullback needs
   if ((rc = fat7_planes(ctx, thin, V1, c_level1, st))) return rc;
   if ((rc = project_u3_planes(ctx, V1, W, st))) return rc;
@@ -324,6 +337,7 @@ int lmb_hisq_links_from_thin(lmb_ctx *ctx, const void *const U[4], const uint64_
     // hisq_links_from_thin! (HISQFullSmearing.jl:284-293)
     const double c_level1[5] = {1.0 / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, 0.0};
     const double c_level2[5] = {1.0 + naik_epsilon / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, -1.0 / 8};
+    if ((rc = fat7_reserve(ctx, false))) return rc;
     if ((rc = pack_links_to(ctx, thin, U, st))) return rc;
     if ((rc = fat7_planes(ctx, thin, lng, c_level1, st))) return rc;
     if ((rc = project_u3_planes(ctx, lng, w, st))) return rc;
@@ -388,6 +402,7 @@ int lmb_hisq_fermion_force(lmb_ctx *ctx, const void *const U[4], const uint64_t 
   if (rc) return rc;
   if ((rc = check_links_arg(ctx, (const void *const *)dU, "force"))) return rc;
   cudaStream_t st = as_stream(stream);
+  if ((rc = fat7_reserve(ctx, true))) return rc;
   // fat / long links for the solve (cached by thin-link pointer + epoch)
   if ((rc = lmb_hisq_links_from_thin(ctx, U, epoch, naik_epsilon, nullptr, nullptr, stream))) return rc;
   // eta = (D^+D)^-1 phi, chi = D eta, in padded scratch fields of the context geometry

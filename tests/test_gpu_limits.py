@@ -145,3 +145,36 @@ def test_directions_take_no_memory_that_is_needed(lmb, orc, monkeypatch, call, p
         assert rd.rel_err(g, w) <= 1e-12
     monkeypatch.setenv("LMB_LIMITS", "workspace=4096")
     assert not _fits(lmb, lambda: call(lmb, orc, precision))
+
+
+def _hisq_gradient(lmb, orc, L):
+    U = _links(lmb, orc.random_su3_links(L, 0.2, 31), 3)
+    dU = [u.similar() for u in U]
+    lmb.hisq_link_pullback_(dU, lmb.HISQDiracCache4D(U, 0.3, -0.083), U, _field(lmb, orc, L, 1, 32, 3),
+                            _field(lmb, orc, L, 1, 33, 3))
+    return [d.gather_matrix() for d in dU]
+
+
+def _hisq_smearing(lmb, orc, L):
+    U, psi = _links(lmb, orc.random_su3_links(L, 0.2, 34), 3), _field(lmb, orc, L, 1, 35, 3)
+    out = psi.similar()
+    lmb.mul_cached_hisq_(out, lmb.HISQDiracCache4D(U, 0.3, -0.083), *U, psi)
+    return [out.gather_matrix()]
+
+
+def _clover_gradient(lmb, orc, L):
+    U = _links(lmb, orc.random_su3_links(L, 0.2, 36), 1)
+    dU = [u.similar() for u in U]
+    lmb.wilson_clover_link_pullback_(dU, lmb.WilsonDiracCloverOperator4D(U, 0.12, 1.0), U, _field(lmb, orc, L, 4, 37, 1),
+                                     _field(lmb, orc, L, 4, 38, 1))
+    return [d.gather_matrix() for d in dU]
+
+
+# The first call on a new context makes each workspace once, at the size of its
+# largest stage: none is freed, which would wait for the device, to be made anew.
+@pytest.mark.parametrize("call", [_hisq_smearing, _hisq_gradient, _clover_gradient,
+                                  lambda lmb, orc, L: _hisq_force(lmb, orc, "double")],
+                         ids=["smearing", "gradient", "clover", "force"])
+def test_first_call_grows_no_workspace(lmb, orc, monkeypatch, call):
+    monkeypatch.setenv("LMB_LIMITS", "growths=0")
+    call(lmb, orc, (4, 4, 4, 4))
