@@ -3,7 +3,6 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include <climits>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -187,12 +186,12 @@ inline int64_t limit_of(const lmb_ctx *ctx, const std::string &key, int64_t most
   return v < most ? v : most;
 }
 
-// whether `bytes` more keep the workspaces within the bound set for them
+// whether `bytes` more keep the workspaces within the bounds set for them
 inline bool workspace_fits(const lmb_ctx *ctx, size_t bytes) {
   if (ctx->limits.empty()) return true;
   int64_t used = (int64_t)bytes;
   for (auto &kv : ctx->buffers) used += (int64_t)kv.second.second;
-  return used <= limit_of(ctx, "workspace", INT64_MAX);
+  return used <= limit_of(ctx, "workspace", INT64_MAX) && ctx->growths <= limit_of(ctx, "growths", INT64_MAX);
 }
 inline bool drop_workspace(lmb_ctx *ctx, const std::string &name) {
   auto it = ctx->buffers.find(name);
@@ -249,7 +248,7 @@ cudaError_t device_malloc(lmb_ctx *ctx, T **p, size_t bytes) {
 inline void *workspace(lmb_ctx *ctx, const std::string &name, size_t bytes) {
   auto it = ctx->buffers.find(name);
   if (it != ctx->buffers.end() && it->second.second >= bytes) return it->second.first;
-  if (drop_workspace(ctx, name) && ctx->growths++ >= limit_of(ctx, "growths", INT_MAX)) return nullptr;
+  if (drop_workspace(ctx, name)) ctx->growths++;
   ctx->spare.erase(name);
   while (!workspace_fits(ctx, bytes))
     if (!release_spare(ctx)) return nullptr;
@@ -265,11 +264,13 @@ inline void *workspace(lmb_ctx *ctx, const std::string &name, size_t bytes) {
 inline void *spare_workspace(lmb_ctx *ctx, const std::string &name, size_t bytes) {
   auto it = ctx->buffers.find(name);
   if (it != ctx->buffers.end() && it->second.second >= bytes) return it->second.first;
-  drop_workspace(ctx, name);
-  ctx->spare.erase(name);
+  const size_t have = it != ctx->buffers.end() ? it->second.second : 0;
   size_t avail = 0, total = 0;
-  if (!workspace_fits(ctx, bytes) || cudaMemGetInfo(&avail, &total) != cudaSuccess || avail < bytes + total / 8)
+  if (!workspace_fits(ctx, bytes - have) || cudaMemGetInfo(&avail, &total) != cudaSuccess ||
+      avail + have < bytes + total / 8)
     return nullptr;
+  if (drop_workspace(ctx, name)) ctx->growths++;
+  ctx->spare.erase(name);
   void *p = nullptr;
   if (cudaMalloc(&p, bytes) != cudaSuccess) {
     cudaGetLastError();

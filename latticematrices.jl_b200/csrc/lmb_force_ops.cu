@@ -42,30 +42,27 @@ SiteTile fat7_tile(const Geom &g, const int *order, int norder) {
 }
 unsigned blocks_of(const SiteTile &t) { return (unsigned)t.n[0] * t.n[1] * t.n[2] * t.n[3]; }
 
+// fields of nine planes a Fat7 map keeps per direction: S and M (M+ and M- with
+// the Lepage term) of the three axes, for the gradient twice
+int64_t fat7_fields(bool lepage, bool gradient) { return (lepage ? 9 : 6) * (gradient ? 2 : 1); }
+
 struct Fat7Launch {
-  int nmu;  // directions per launch
-  int64_t per_mu;
+  int nmu;         // directions per launch
+  int64_t per_mu;  // stride of their workspaces
+  double2 *work;   // nullptr: out of memory
 };
 // Directions per launch.  One direction's three axes give V / 128 x 3 blocks;
 // below 64 Ki sites that is less than about four waves of the 148 SMs, and
 // the four directions share a launch (their workspaces then hold at most
-// 700 MB); larger lattices keep one direction's workspace.
-Fat7Launch fat7_launch(const Geom &g, int fields) {
-  return Fat7Launch{g.V <= (1 << 16) ? 4 : 1, (int64_t)fields * 9 * g.V};
-}
-// fields of nine planes per direction: S and M (M+ and M- with the Lepage
-// term) of the three axes, for the gradient twice
-int fat7_fields(bool lepage, bool gradient) { return (lepage ? 9 : 6) * (gradient ? 2 : 1); }
-double2 *fat7_workspace(lmb_ctx *ctx, const Fat7Launch &l) {
-  return (double2 *)workspace(ctx, "fat7", sizeof(double2) * l.nmu * l.per_mu);
-}
-// A chain's largest stage is its second level's, with the Lepage term; asked
-// for first, so that the first level's is not freed for it (first smearing and
-// link gradient of a new operator: see hisq_links_from_thin and
-// hisq_pullback_planes)
-int fat7_reserve(lmb_ctx *ctx, bool gradient) {
-  if (fat7_workspace(ctx, fat7_launch(ctx->g, fat7_fields(true, gradient)))) return LMB_OK;
-  return fail(ctx, LMB_ERR_CUDA, "out of device memory (Fat7 stages)");
+// 700 MB).  Larger lattices, and those whose four workspaces find no memory,
+// keep one direction's.  `fields`: of the largest map of the call, which asks
+// once, so that no level's workspace is freed for the next one's.
+Fat7Launch fat7_launch(lmb_ctx *ctx, int64_t fields) {
+  const int64_t per_mu = fields * 9 * ctx->g.V;
+  const size_t bytes = sizeof(double2) * per_mu;
+  double2 *work = ctx->g.V <= (1 << 16) ? (double2 *)spare_workspace(ctx, "fat7", 4 * bytes) : nullptr;
+  if (work) return Fat7Launch{4, per_mu, work};
+  return Fat7Launch{1, per_mu, (double2 *)workspace(ctx, "fat7", bytes)};
 }
 
 // block shapes of a stage for the directions mu0 .. mu0 + nmu - 1, and the
@@ -109,12 +106,11 @@ void fat7_sum(lmb_ctx *ctx, const Fat7Launch &l, const double2 *U, double2 *out,
 }
 
 // V = Fat7(U) with coefficients (c1, c3, c5, c7, cLepage)
-int fat7_planes(lmb_ctx *ctx, const double2 *U, double2 *V, const double *coef, cudaStream_t st) {
+int fat7_planes(lmb_ctx *ctx, const Fat7Launch &l, const double2 *U, double2 *V, const double *coef,
+                cudaStream_t st) {
   const int64_t F3 = 27 * ctx->g.V;  // the three axes' fields
   const bool lepage = coef[4] != 0.0;
-  const Fat7Launch l = fat7_launch(ctx->g, fat7_fields(lepage, false));
-  double2 *work = fat7_workspace(ctx, l);
-  if (!work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing staples)");
+  double2 *work = l.work;
   const Fat7Field f{U, work, work + F3, lepage ? work + 2 * F3 : work + F3, coef[1]};
   for (int mu = 0; mu < 4; mu += l.nmu) {
     if (lepage)
@@ -164,13 +160,11 @@ int install_links(lmb_ctx *ctx, int which, cudaStream_t st) {
 
 // dU += d/dU Re<dV, Fat7(U)>: the staples of U and of dV, the Fat7 map of dV
 // onto its own direction, and the transports' links
-int fat7_pullback_planes(lmb_ctx *ctx, const double2 *U, const double2 *dV, double2 *dU, const double *coef,
-                         cudaStream_t st) {
+int fat7_pullback_planes(lmb_ctx *ctx, const Fat7Launch &l, const double2 *U, const double2 *dV, double2 *dU,
+                         const double *coef, cudaStream_t st) {
   const int64_t F3 = 27 * ctx->g.V;
   const bool lepage = coef[4] != 0.0;
-  const Fat7Launch l = fat7_launch(ctx->g, fat7_fields(lepage, true));
-  double2 *work = fat7_workspace(ctx, l);
-  if (!work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (force staples)");
+  double2 *work = l.work;
   const Fat7Field fu{U, work, work + F3, lepage ? work + 4 * F3 : work + F3, 0.0};
   const Fat7Field fg{dV, work + 2 * F3, work + 3 * F3, lepage ? work + 5 * F3 : work + 3 * F3, coef[1]};
   for (int mu = 0; mu < 4; mu += l.nmu) {
@@ -200,9 +194,10 @@ int hisq_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_DOU
   const double c_level1[5] = {1.0 / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, 0.0};
   const double c_level2[5] = {1.0 + naik_epsilon / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, -1.0 / 8};
   int rc;
-  if ((rc = fat7_reserve(ctx, true))) return rc;
+  const Fat7Launch l = fat7_launch(ctx, fat7_fields(true, true));
+  if (!l.work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (force staples)");
   // recompute the smearing levels the pullback needs
-  if ((rc = fat7_planes(ctx, thin, V1, c_level1, st))) return rc;
+  if ((rc = fat7_planes(ctx, l, thin, V1, c_level1, st))) return rc;
   if ((rc = project_u3_planes(ctx, V1, W, st))) return rc;
   // Dirac outer products
   const double fc = coefficient / 2, lc = -coefficient * (1.0 + naik_epsilon) / 48.0;
@@ -212,13 +207,13 @@ int hisq_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_DOU
   LMB_CUDA(ctx, cudaMemsetAsync(dW, 0, L36, st));
   naik_pullback_kernel<<<grid_for(4 * n, kSmearThreads), kSmearThreads, 0, st>>>(dW, dL, W, ctx->g);
   LMB_CHECK_LAUNCH(ctx);
-  if ((rc = fat7_pullback_planes(ctx, W, dX, dW, c_level2, st))) return rc;
+  if ((rc = fat7_pullback_planes(ctx, l, W, dX, dW, c_level2, st))) return rc;
   // U(3) projection -> dV1
   LMB_CUDA(ctx, cudaMemsetAsync(dV1, 0, L36, st));
   u3_pullback_kernel<<<grid_for(4 * n, 64), 64, 0, st>>>(dV1, dW, V1, n);
   LMB_CHECK_LAUNCH(ctx);
   // level-1 Fat7 -> thin links
-  return fat7_pullback_planes(ctx, thin, dV1, dU, c_level1, st);
+  return fat7_pullback_planes(ctx, l, thin, dV1, dU, c_level1, st);
 }
 
 // grad (36 planes) = d/dU [coef Re<dr, D_clover(U) psi>]
@@ -230,11 +225,13 @@ int clover_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_D
   LMB_CHECK_LAUNCH(ctx);
   if (csw == 0.0) return LMB_OK;
   // the inserted links of all planes at once (1728 B per site), or of one
-  // plane at a time on lattices above 4 Mi sites: with the packed H that is
-  // less memory than the six full cotangents
-  const int np = n <= (1 << 22) ? 6 : 1;
+  // plane at a time on lattices above 4 Mi sites and where those of six find
+  // no memory: with the packed H that is less than the six full cotangents
+  const size_t plane = sizeof(double2) * 18 * n;
   double2 *H = (double2 *)workspace(ctx, "force_H", sizeof(double2) * 6 * kAntiPlanes * n);
-  double2 *W = (double2 *)workspace(ctx, "force_insert", sizeof(double2) * 18 * np * n);
+  double2 *W = n <= (1 << 22) ? (double2 *)spare_workspace(ctx, "force_insert", 6 * plane) : nullptr;
+  const int np = W ? 6 : 1;
+  if (!W) W = (double2 *)workspace(ctx, "force_insert", plane);
   if (!H || !W) return fail(ctx, LMB_ERR_CUDA, "out of device memory (clover force)");
   clover_cotangent_kernel<<<grid_for(n, 128), 128, 0, st>>>(H, dr, psi, ctx->g, -kappa * csw * coefficient);
   LMB_CHECK_LAUNCH(ctx);
@@ -278,8 +275,10 @@ int lmb_hisq_fat7(lmb_ctx *ctx, const void *const U[4], const double coefficient
   double2 *in = (double2 *)workspace(ctx, "smear_in", sizeof(double2) * 36 * n);
   double2 *out = (double2 *)workspace(ctx, "smear_out", sizeof(double2) * 36 * n);
   if (!in || !out) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing)");
+  const Fat7Launch l = fat7_launch(ctx, fat7_fields(coefficients[4] != 0.0, false));
+  if (!l.work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing staples)");
   if ((rc = pack_links_to(ctx, in, U, st))) return rc;
-  if ((rc = fat7_planes(ctx, in, out, coefficients, st))) return rc;
+  if ((rc = fat7_planes(ctx, l, in, out, coefficients, st))) return rc;
   return unpack_links_from(ctx, V, out, st);
 }
 
@@ -337,11 +336,12 @@ int lmb_hisq_links_from_thin(lmb_ctx *ctx, const void *const U[4], const uint64_
     // hisq_links_from_thin! (HISQFullSmearing.jl:284-293)
     const double c_level1[5] = {1.0 / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, 0.0};
     const double c_level2[5] = {1.0 + naik_epsilon / 8, 1.0 / 16, 1.0 / 64, 1.0 / 384, -1.0 / 8};
-    if ((rc = fat7_reserve(ctx, false))) return rc;
+    const Fat7Launch l = fat7_launch(ctx, fat7_fields(true, false));
+    if (!l.work) return fail(ctx, LMB_ERR_CUDA, "out of device memory (smearing staples)");
     if ((rc = pack_links_to(ctx, thin, U, st))) return rc;
-    if ((rc = fat7_planes(ctx, thin, lng, c_level1, st))) return rc;
+    if ((rc = fat7_planes(ctx, l, thin, lng, c_level1, st))) return rc;
     if ((rc = project_u3_planes(ctx, lng, w, st))) return rc;
-    if ((rc = fat7_planes(ctx, w, fat, c_level2, st))) return rc;
+    if ((rc = fat7_planes(ctx, l, w, fat, c_level2, st))) return rc;
     if ((rc = naik_planes(ctx, w, lng, st))) return rc;
     if ((rc = install_links(ctx, LMB_LINKS_FAT, st))) return rc;
     if ((rc = install_links(ctx, LMB_LINKS_LONG, st))) return rc;
@@ -402,7 +402,9 @@ int lmb_hisq_fermion_force(lmb_ctx *ctx, const void *const U[4], const uint64_t 
   if (rc) return rc;
   if ((rc = check_links_arg(ctx, (const void *const *)dU, "force"))) return rc;
   cudaStream_t st = as_stream(stream);
-  if ((rc = fat7_reserve(ctx, true))) return rc;
+  // the gradient's workspace, which the smearing then shares
+  if (!fat7_launch(ctx, fat7_fields(true, true)).work)
+    return fail(ctx, LMB_ERR_CUDA, "out of device memory (force staples)");
   // fat / long links for the solve (cached by thin-link pointer + epoch)
   if ((rc = lmb_hisq_links_from_thin(ctx, U, epoch, naik_epsilon, nullptr, nullptr, stream))) return rc;
   // eta = (D^+D)^-1 phi, chi = D eta, in padded scratch fields of the context geometry

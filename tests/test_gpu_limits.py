@@ -178,3 +178,18 @@ def _clover_gradient(lmb, orc, L):
 def test_first_call_grows_no_workspace(lmb, orc, monkeypatch, call):
     monkeypatch.setenv("LMB_LIMITS", "growths=0")
     call(lmb, orc, (4, 4, 4, 4))
+
+
+# One direction's (one plane's) workspace where those of all four (six) find no
+# memory: bytes per site of the fields a call cannot do without, and 64 KiB of
+# small ones.  All together would take 5184, 10368 - 2592 and 1440 more.  The
+# stages are the same; the sums into a link run in another order.
+@pytest.mark.parametrize("call,site", [(_hisq_smearing, 2 * 576 + 1296 + 2 * 48),
+                                       (_hisq_gradient, 8 * 576 + 2592 + 2 * 48),
+                                       (_clover_gradient, 2 * 576 + 2 * 192 + 480 + 288)])
+@pytest.mark.parametrize("L", [(4, 4, 6, 8), (5, 3, 7, 9)])
+def test_gradients_in_less_memory(lmb, orc, monkeypatch, call, site, L):
+    want = call(lmb, orc, L)
+    monkeypatch.setenv("LMB_LIMITS", f"workspace={int(np.prod(L)) * site + 65536}")
+    for g, w in zip(call(lmb, orc, L), want):
+        assert rd.rel_err(g, w) <= 1e-13
