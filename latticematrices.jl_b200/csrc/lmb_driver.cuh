@@ -31,8 +31,8 @@ int op_unpack_out(lmb_ctx *ctx, const Op &, void *dst, const Field<PS, NC> &f, c
 template <int PS, class Op> bool op_reserve(lmb_ctx *, const Op &) { return true; }
 
 // all iterations up to the next status change in one launch (lmb_small.cuh):
-// LMB_OK or an error; kNotSmall where the operator or the lattice has no such
-// kernel
+// LMB_OK or an error; kNotSmall, with nothing done, where the operator or the
+// lattice has no such kernel or its launch or workspace is refused
 constexpr int kNotSmall = 1;
 constexpr int kSmallIters = 1000;
 template <class Op, int PS, int PX, int NC>
@@ -363,7 +363,8 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
   };
   while (hs->status == ST_RUNNING) {
     const int it0 = hs->iter;
-    const int small = prm->profile ? kNotSmall : op_cg_small(ctx, op, p, rl, tl, xl, st);
+    // (not asked again once the staged kernels run)
+    const int small = prm->profile || depth ? kNotSmall : op_cg_small(ctx, op, p, rl, tl, xl, st);
     if (small != kNotSmall && small != LMB_OK) return small;
     if (small == LMB_OK) nl++;
     if (small == kNotSmall && !depth && !make_ring())

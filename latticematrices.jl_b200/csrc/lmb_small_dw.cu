@@ -115,8 +115,7 @@ int op_cg_small(lmb_ctx *ctx, const DWPolicy &op, const Field<PS, 12> &p, const 
                 const Field<PS, 12> &t, const Field<PX, 12> &x, cudaStream_t st) {
   if (!ctx->persistent) return kNotSmall;
   Field<PS, 12> mid;
-  if (!DWPolicy::make_tmp(ctx, mid))
-    return fail(ctx, LMB_ERR_CUDA, "out of device memory (domain-wall workspace)");
+  if (!DWPolicy::make_tmp(ctx, mid)) return kNotSmall;
   const DWParams d = op.params(ctx);
   const LinkSet &ls = ctx->links[LMB_LINKS_THIN];
   if (ls.recon(PS))

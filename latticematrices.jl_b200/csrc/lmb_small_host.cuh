@@ -21,7 +21,9 @@ template <int PS, int PX, class Op>
 int small_cg(lmb_ctx *ctx, const Op &op, const Field<PS, Op::NC> &p, const Field<PS, Op::NC> &r,
              const Field<PS, Op::NC> &t, const Field<PX, Op::NC> &x, cudaStream_t st) {
   auto kern = small_cg_kernel<PS, PX, Op>;
-  const int64_t resident = (int64_t)small_resident((const void *)kern) * std::max(1, ctx->sm_count);
+  int64_t per_sm = limit_of(ctx, "blocks", INT64_MAX);  // set: assumed, not asked for
+  if (per_sm == INT64_MAX) per_sm = small_resident((const void *)kern);
+  const int64_t resident = per_sm * std::max(1, ctx->sm_count);
   // A phase of this kernel costs its barrier and as many tile latencies as a
   // block has tiles, a stage of the staged solver its launch and its longest
   // thread, then its bytes.  The line between them lies at a number of tiles
@@ -42,7 +44,7 @@ int small_cg(lmb_ctx *ctx, const Op &op, const Field<PS, Op::NC> &p, const Field
   // every block is resident (a cooperative launch): the barriers can be met
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, resident);
   char *ws = (char *)workspace(ctx, "small_cg", 256 + 2 * sizeof(double) * resident);
-  if (!ws) return fail(ctx, LMB_ERR_CUDA, "out of device memory (small-lattice solver)");
+  if (!ws) return kNotSmall;
   LMB_CUDA(ctx, cudaMemsetAsync(ws, 0, 256, st));
   Geom g = ctx->g;
   Op o = op;
@@ -52,7 +54,14 @@ int small_cg(lmb_ctx *ctx, const Op &op, const Field<PS, Op::NC> &p, const Field
   SmallGrid gr{(unsigned *)ws, (double *)(ws + 256)};
   int iters = kSmallIters;
   void *args[] = {&g, &o, &fp, &fr, &ft, &fx, &state, &gr, &iters};
-  LMB_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kSmallThreads), args, 0, st));
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kSmallThreads), args, 0, st);
+  // refused before anything ran: the device cannot hold the grid at once (a
+  // process that was given a share of its SMs, say), or takes no such launch
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorNotPermitted) {
+    cudaGetLastError();
+    return kNotSmall;
+  }
+  LMB_CUDA(ctx, e);
   return LMB_OK;
 }
 

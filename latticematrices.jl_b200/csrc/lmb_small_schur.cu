@@ -100,8 +100,7 @@ int small_schur(lmb_ctx *ctx, const SchurPolicy &op, const G &U, const Field<PS,
                 const Field<PS, 12> &t, const Field<PX, 12> &x, cudaStream_t st) {
   typedef typename Real<PS>::type R;
   Field<PS, 12> mid;
-  if (!SchurPolicy::make_tmp(ctx, mid))
-    return fail(ctx, LMB_ERR_CUDA, "out of device memory (even/odd workspace)");
+  if (!SchurPolicy::make_tmp(ctx, mid)) return kNotSmall;
   const Clover<PS> A = eo_clover_view<PS>(ctx, 0), Ai = eo_clover_view<PS>(ctx, 1);
   const R mk2 = (R)(-op.kappa * op.kappa);
   if (op.clover) return small_cg(ctx, SmallSchur<PS, G, true>{U, A, Ai, mk2, mid}, p, r, t, x, st);

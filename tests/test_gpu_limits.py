@@ -193,3 +193,32 @@ def test_gradients_in_less_memory(lmb, orc, monkeypatch, call, site, L):
     monkeypatch.setenv("LMB_LIMITS", f"workspace={int(np.prod(L)) * site + 65536}")
     for g, w in zip(call(lmb, orc, L), want):
         assert rd.rel_err(g, w) <= 1e-13
+
+
+# The one-launch solver of small lattices, with a grid larger than the device can
+# hold at once (refused by the host before anything runs) and with no memory for
+# its barrier: the solve takes the staged kernels, three launches an iteration.
+@pytest.mark.parametrize("limits", ["blocks=64", "workspace"])
+def test_refused_cooperative_launch(lmb, orc, monkeypatch, limits):
+    L, rtol = (16, 12, 12, 12), 1e-9
+    U, b = orc.random_su3_links(L, 0.25, 41), orc.gaussian_field(L, 3, 4, 42)
+    bd = lmb.LatticeMatrix.from_array(b, nw=1, phases=PHASES)
+
+    def run():
+        x, D = bd.similar(), lmb.WilsonDiracOperator4D(_links(lmb, U, 1), 0.12)
+        return lmb.cg_(x, lmb.DdagDOp(D, bd.similar()), bd, rtol=rtol), x
+    one, _ = run()
+    assert one.kernel_launches < one.iterations
+    if limits == "workspace":  # what the staged kernels take, to 4 KiB
+        def staged(n):
+            monkeypatch.setenv("LMB_LIMITS", f"directions=1,workspace={n}")
+            return _fits(lmb, run)
+        monkeypatch.setenv("LMB_PERSISTENT", "0")
+        limits = f"directions=1,workspace={_least(staged)}"
+        monkeypatch.setenv("LMB_PERSISTENT", "1")
+    monkeypatch.setenv("LMB_LIMITS", limits)
+    res, x = run()
+    assert res.converged and res.iterations == one.iterations
+    assert res.kernel_launches >= 3 * res.iterations
+    op = orc.Operator(orc.OP_WILSON, U, L, kappa=0.12)
+    assert rd.rel_err(op.ddagd(np.asfortranarray(x.gather_matrix())), b) <= 1.05 * rtol
