@@ -224,15 +224,17 @@ int clover_pullback_planes(lmb_ctx *ctx, const double2 *thin, const Field<PREC_D
   wilson_outer_product_kernel<<<grid_for(n, 128), 128, 0, st>>>(grad, dr, psi, ctx->g, -kappa * coefficient);
   LMB_CHECK_LAUNCH(ctx);
   if (csw == 0.0) return LMB_OK;
-  // the inserted links of all planes at once (1728 B per site), or of one
-  // plane at a time on lattices above 4 Mi sites and where those of six find
-  // no memory: with the packed H that is less than the six full cotangents
-  const size_t plane = sizeof(double2) * 18 * n;
-  double2 *H = (double2 *)workspace(ctx, "force_H", sizeof(double2) * 6 * kAntiPlanes * n);
-  double2 *W = n <= (1 << 22) ? (double2 *)spare_workspace(ctx, "force_insert", 6 * plane) : nullptr;
-  const int np = W ? 6 : 1;
-  if (!W) W = (double2 *)workspace(ctx, "force_insert", plane);
-  if (!H || !W) return fail(ctx, LMB_ERR_CUDA, "out of device memory (clover force)");
+  // the packed H of the six planes and the inserted links of all of them at once
+  // (1728 B per site), or of one plane at a time on lattices above 4 Mi sites and
+  // where those of six find no memory: together less than the six full cotangents.
+  // One workspace: an allocation takes 0.3 ms of a first call
+  const int64_t plane = 18 * n, packed = 6 * kAntiPlanes * n;
+  double2 *H = nullptr;
+  if (n <= (1 << 22)) H = (double2 *)spare_workspace(ctx, "force_clover", sizeof(double2) * (packed + 6 * plane));
+  const int np = H ? 6 : 1;
+  if (!H) H = (double2 *)workspace(ctx, "force_clover", sizeof(double2) * (packed + plane));
+  if (!H) return fail(ctx, LMB_ERR_CUDA, "out of device memory (clover force)");
+  double2 *W = H + packed;
   clover_cotangent_kernel<<<grid_for(n, 128), 128, 0, st>>>(H, dr, psi, ctx->g, -kappa * csw * coefficient);
   LMB_CHECK_LAUNCH(ctx);
   Fat7Tiles tl;
