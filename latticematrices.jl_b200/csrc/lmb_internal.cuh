@@ -30,10 +30,16 @@ unsigned resident_grid(const lmb_ctx *ctx, K kern) {
   return (unsigned)(resident_blocks_per_sm((const void *)kern) * (ctx->sm_count > 0 ? ctx->sm_count : 1));
 }
 
-// whether `threads` threads of a pair kernel (three blocks of 128 per SM) fill at
-// least num / den of the device's resident blocks
-inline bool fills_device(const lmb_ctx *ctx, int64_t threads, int num, int den) {
-  return den * threads >= (int64_t)num * 3 * kDslashThreads * (ctx->sm_count > 0 ? ctx->sm_count : 1);
+// blocks of a kernel of kDslashThreads threads, and the device's slots for them
+// at `per_sm` resident blocks per SM: whether the blocks fill num / den of the
+// slots, and of those of their waves
+inline bool fills_device(const lmb_ctx *ctx, int64_t threads, int per_sm, int num, int den) {
+  return den * threads >= (int64_t)num * per_sm * kDslashThreads * (ctx->sm_count > 0 ? ctx->sm_count : 1);
+}
+inline bool fills_waves(const lmb_ctx *ctx, int64_t threads, int per_sm, int num, int den) {
+  const int64_t slots = (int64_t)per_sm * (ctx->sm_count > 0 ? ctx->sm_count : 1);
+  const int64_t blocks = grid_for(threads, kDslashThreads), waves = (blocks + slots - 1) / slots;
+  return den * blocks >= num * waves * slots;
 }
 
 inline int check_prec(lmb_ctx *ctx, int prec) {

@@ -20,15 +20,22 @@ struct DWPolicy {
   }
   static bool one_pass(const lmb_ctx *ctx) { return ctx->dw_L5 <= kDslashThreads && !ctx->dw_two_pass; }
   // FP32 / int16: two slices per thread (every pair of slices is one 256-bit
-  // word of a plane when L5 is even), on lattices that give the half as many
-  // threads enough blocks.  Solves, one site -> pairs: int16 8^3x12x8 (192
-  // blocks of 444) 11.0 -> 11.1 ms, 8^3x16x8 (256) 14.5 -> 13.8, 12^3x16^2
-  // (864) 55.7 -> 47.1; FP32 8^3x16x8 14.1 -> 15.4, 8^2x12^2x10 (360) 17.7 ->
-  // 15.8, 8^2x12x16x12 (576, two waves) 24.9 -> 25.6, 8x12^2x16x12 (864) 33.0
-  // -> 30.0.
+  // word of a plane when L5 is even), where half as many threads still fill the
+  // device.  Solves at L5 = 12 on 148 SMs by the blocks of pairs, one site ->
+  // pairs, ms.
+  // FP32, three blocks per SM (444 slots): from two thirds of the slots of its
+  // waves on, so not between one wave and 1.33.  192 blocks 9.9 -> 10.3, 300 14.7
+  // -> 14.0, 432 19.3 -> 17.0, 480 22.3 -> 24.1, 540 20.0 -> 21.8, 576 24.6 ->
+  // 25.6, 630 25.8 -> 24.7, 864 33.7 -> 30.2, 945 35.9 -> 35.6, 1080 40.8 -> 40.0,
+  // 1296 48.3 -> 44.3, 1728 70.1 -> 65.7.
+  // int16, four (592): from 3/8 of them on, 222 blocks.  192 9.6 -> 9.8, 300 14.5
+  // -> 13.8, 432 19.1 -> 17.1, 480 22.4 -> 21.8, 576 25.8 -> 21.7, 630 25.6 ->
+  // 23.3, 864 32.5 -> 27.2, 1296 45.1 -> 39.8, 1728 65.2 -> 54.7.
   template <int P> static bool pairs(const lmb_ctx *ctx) {
+    const int64_t threads = ctx->g.V * (ctx->dw_L5 / 2);
+    constexpr int per_sm = DWPairBlocks<Field<P, 12>>::value;
     return one_pass(ctx) && ctx->pair_sites && ctx->adj_sites && ctx->dw_L5 % 2 == 0 &&
-           fills_device(ctx, ctx->g.V * (ctx->dw_L5 / 2), P == PREC_HALF ? 2 : 3, 4);
+           (P == PREC_HALF ? fills_device(ctx, threads, per_sm, 3, 8) : fills_waves(ctx, threads, per_sm, 2, 3));
   }
   // the field between two passes (the two-pass launches, the small-lattice D5^+)
   template <int P> static bool make_tmp(lmb_ctx *ctx, Field<P, 12> &f) {

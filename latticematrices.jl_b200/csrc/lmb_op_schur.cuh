@@ -76,6 +76,16 @@ struct SchurPolicy {
     }
     return ensure_eo_copies(ctx, prec, clover, st);
   }
+  // int16: two checkerboard neighbours per thread, which stay in one row when the
+  // row holds an even number of them, from half of the 444 resident blocks on.
+  // Solves on 148 SMs by the blocks of pairs, one site -> pairs, ms: clover 160
+  // 7.28 -> 7.36, 200 8.55 -> 8.25, 240 9.80 -> 9.54, 420 14.8 -> 13.1, 450 15.2 ->
+  // 14.9, 540 16.0 -> 15.8, 756 23.8 -> 21.2, 1372 39.4 -> 37.0; Wilson 200 4.46 ->
+  // 4.54, 240 4.72 -> 4.51, 420 7.03 -> 6.49, 540 8.03 -> 7.80, 756 10.7 -> 9.9.
+  // (FP32 pairs fill the registers with their loads: 24^3x48 clover 50.5 -> 53.6.)
+  static bool pairs(const lmb_ctx *ctx) {
+    return ctx->pair_sites && ctx->adj_sites && ctx->g.L[0] % 4 == 0 && fills_device(ctx, ctx->g.V / 4, 3, 1, 2);
+  }
   // the odd half field between the two hops
   template <int P> static bool make_tmp(lmb_ctx *ctx, Field<P, 12> &t) {
     return make_field(ctx, P == PREC_DOUBLE ? "eo_t_d" : (P == PREC_SINGLE ? "eo_t_s" : "eo_t_h"), t, ctx->g.V / 2);
@@ -88,13 +98,7 @@ struct SchurPolicy {
     const unsigned grid = grid_for(ctx->g.V / 2, kDslashThreads);
     const EpiStoreFollow<P, Epi> e1{t, epi};
     if constexpr (P == PREC_HALF) {
-      // pairs of checkerboard neighbours stay in one row when the row holds
-      // an even number of them.  int16 only: at 24^3x48 clover its solve takes
-      // 35.3 ms on pairs against 40.2 ms, the FP32 one, whose loads already
-      // fill the registers, 53.6 against 50.5 ms.  And from half the resident
-      // blocks on: clover 16^4 (128 blocks of 444) 6.3 -> 6.6 ms, 16^2x24^2
-      // (288) 10.4 -> 9.8
-      if (ctx->pair_sites && ctx->adj_sites && ctx->g.L[0] % 4 == 0 && fills_device(ctx, ctx->g.V / 4, 1, 2)) {
+      if (pairs(ctx)) {
         const unsigned g2 = grid_for(ctx->g.V / 4, kDslashThreads);
         eo_hop_pair_kernel<DAG, 0, true, CL><<<g2, kDslashThreads, 0, st>>>(ctx->g, 1, in, in, U, A, Ai, 0.f, 1.f, e1);
         eo_hop_pair_kernel<DAG, 2, false, CL><<<g2, kDslashThreads, 0, st>>>(ctx->g, 0, t, in, U, A, Ai, 1.f,
