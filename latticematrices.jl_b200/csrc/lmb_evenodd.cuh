@@ -211,13 +211,21 @@ LMB_D void clover_apply(const C &A, int64_t s, Cx<R> *v) {
   }
 }
 
+// Resident blocks per SM: as the Wilson stencils (SiteMinBlocks), but two where
+// FP64 links keep 18 reals and the 168 registers of three spill 130 bytes.
+// Solves with one, three and two of them asked for, ms: clover 12^2x16^2 5.6, 5.6,
+// 4.8, 16^3x32 19.4, 20.2, 15.3, 24^4 45.0, 36.9, 34.8, 24^3x48 90.7, 79.1, 71.3;
+// Wilson 16^3x32 10.0, 9.5, 7.3, 24^3x32 28.3, 22.8, 21.6.
+template <typename R, class G> struct EoMinBlocks { static constexpr int value = SiteMinBlocks<R>::value; };
+template <> struct EoMinBlocks<double, Gauge<PREC_DOUBLE>> { static constexpr int value = 2; };
+
 // Sites of parity p (one thread per checkerboard index; links and clover
 // blocks parity-ordered):
 //   v = c1 W(x) [WMODE 1]  or  c1 A(x) W(x) [WMODE 2]  (W: parity p)
 //     + c2 (H in)(x)        (H^+ when DAG; in: parity 1 - p)
 //   out = A^-1(x) v when AINV, else v.     CL = false: A = 1.
 template <typename R, int DAG, int WMODE, bool AINV, bool CL, class SF, class G, class C, class Epi>
-__global__ void __launch_bounds__(kDslashThreads, SiteMinBlocks<R>::value)
+__global__ void __launch_bounds__(kDslashThreads, EoMinBlocks<R, G>::value)
     eo_hop_kernel(const Geom g, const int p, const SF in, const SF W, const G U, const C A, const C Ainv,
                   const R c1, const R c2, Epi epi) {
   if (epi.skip()) return;
