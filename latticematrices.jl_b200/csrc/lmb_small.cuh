@@ -417,7 +417,6 @@ struct SmallStaggered {
 struct SmallGrid {
   unsigned *arrived;  // zeroed before the launch
   double *partials;   // 2 gridDim.x
-  int spins;          // polls of the counter until a block gives up
 };
 constexpr int kSmallSpins = 1 << 21;  // about two seconds
 
@@ -454,7 +453,7 @@ LMB_D bool small_grid_sum(const SmallGrid &gr, unsigned &epoch, double x, double
     unsigned seen;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(gr.arrived) : "memory");
-    } while (seen < goal && ++n < gr.spins);
+    } while (seen < goal && ++n < kSmallSpins);
     met = seen >= goal;
   }
   __syncthreads();

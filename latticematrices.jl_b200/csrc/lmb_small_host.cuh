@@ -61,7 +61,7 @@ int small_cg(lmb_ctx *ctx, const Op &op, const Field<PS, Op::NC> &p, const Field
   Field<PS, Op::NC> fp = p, fr = r, ft = t;
   Field<PX, Op::NC> fx = x;
   CGState *state = ctx->st_dev;
-  SmallGrid gr{(unsigned *)ws, (double *)(ws + 256), (int)limit_of(ctx, "spins", kSmallSpins)};
+  SmallGrid gr{(unsigned *)ws, (double *)(ws + 256)};
   int iters = kSmallIters;
   void *args[] = {&g, &o, &fp, &fr, &ft, &fx, &state, &gr, &iters};
   const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kSmallThreads), args, 0, st);

@@ -224,26 +224,6 @@ def test_refused_cooperative_launch(lmb, orc, monkeypatch, limits):
     assert rd.rel_err(op.ddagd(np.asfortranarray(x.gather_matrix())), b) <= 1.05 * rtol
 
 
-# A barrier of the one-launch solver that is polled once: the blocks that come
-# before the last give up and return, those that wait for them do so at the next
-# barrier, and the solve ends with an error.  The context stays usable.
-@pytest.mark.parametrize("precision", ["double", "half"])
-def test_barrier_that_runs_out(lmb, orc, monkeypatch, precision):
-    L = (8, 8, 8, 8)
-    U, b = orc.random_su3_links(L, 0.25, 51), orc.gaussian_field(L, 3, 4, 52)
-    monkeypatch.setenv("LMB_LIMITS", "spins=1")
-    D = lmb.WilsonDiracOperator4D(_links(lmb, U, 1), 0.12)
-    bd = lmb.LatticeMatrix.from_array(b, nw=1, phases=PHASES)
-    with pytest.raises(lmb.LMBError, match="grid barrier"):
-        lmb.cg_(bd.similar(), lmb.DdagDOp(D, bd.similar()), bd, precision=precision)
-    out = bd.similar()
-    lmb.mul_(out, D, bd)
-    assert rd.rel_err(out.gather_matrix(), orc.wilson(U, b, 0.12, PHASES)) <= 1e-13
-    monkeypatch.delenv("LMB_LIMITS")
-    D, x = lmb.WilsonDiracOperator4D(_links(lmb, U, 1), 0.12), bd.similar()
-    assert lmb.cg_(x, lmb.DdagDOp(D, bd.similar()), bd, precision=precision).converged
-
-
 # Which solver runs, told by the launches: one for all iterations up to a reliable
 # update, or three an iteration.
 @pytest.mark.parametrize("tiles", [0, 100])
