@@ -309,6 +309,7 @@ void lmb_destroy(lmb_ctx *ctx) {
   for (auto &bl : ctx->batch_links) {
     cudaFree(bl.d12);
     cudaFree(bl.f12);
+    cudaFree(bl.h12);
   }
   release_site_caches(ctx);
   dist_release(ctx);
