@@ -616,11 +616,11 @@ def run_hisq(args):
     out = {"workload": "HISQ smearing + staggered D'D CG, %dx%dx%dx%d, m 0.01" % L,
            "smear_s": t_smear}
     # algorithmic bytes per site (each link matrix once: 4 fat + 4 Naik x 18
-    # reals; K1 links + in + out, K2 links + in + p + r (rw) + x (rw, once in
-    # X_UPDATE iterations)): FP32 / FP64 156 and 171 reals; int16 links
-    # 8 x 36 B, spinor 16 B + 4 B norm, x FP32 24 B
-    kbytes = {"single": (156 * 4, 171 * 4), "double": (156 * 8, 171 * 8),
-              "half": (288 + 2 * 20, 288 + 4 * 20 + 2 * 24 // X_UPDATE)}
+    # reals; K1 links + in + out, K2 links + in + p + r (rw) + x (rw, FP64 once
+    # in X_UPDATE iterations)): FP32 156 and 180 reals, FP64 156 and 171; int16
+    # links 8 x 36 B, spinor 16 B + 4 B norm, x FP32 24 B
+    kbytes = {"single": (156 * 4, 180 * 4), "double": (156 * 8, 171 * 8),
+              "half": (288 + 2 * 20, 288 + 4 * 20 + 2 * 24)}
     for prec in ("single", "half", "double"):
         lmb.clear_matrix_(x)
         lmb.cg_(x, A, b, rtol=1e-10, precision=prec, maxiter=args.maxiter)
@@ -935,17 +935,18 @@ def run_dw(args):
                                          maxiter=args.maxiter, profile=True), st)
         k1 = res.dslash_ms / max(res.dslash_launches, 1)
         k2 = res.update_ms / max(res.update_launches, 1)
-        sp, xb = spinor_bytes(prec), x_bytes(prec)
+        sp = spinor_bytes(prec)
+        xb = 2 * x_bytes(prec) // (1 if prec == "double" else X_UPDATE)
         links = 4 * res.link_reals * REAL_BYTES[prec] / L5  # 4D links shared by L5 slices
         # bytes per 5D site the two-pass kernels move (each operand once):
         #  K1 = D5 p:  Y = B p + C F p (p, Y), stencil (Y, p, out, links)
         #  K2 = D5^+ t + CG update: stencil (t, Z, links), local (t, Z, p,
-        #       r rw, x rw once in X_UPDATE iterations)
+        #       r rw, x rw: FP32 and int16 once in X_UPDATE iterations)
         k1_b = 5 * sp + links
-        k2_b = 7 * sp + 2 * xb // X_UPDATE + links
+        k2_b = 7 * sp + xb + links
         # the operator's compulsory bytes (a one-pass kernel): in, out, links
         k1_min = 2 * sp + links
-        k2_min = 4 * sp + 2 * xb // X_UPDATE + links
+        k2_min = 4 * sp + xb + links
         out[prec] = {"time_s": t, "iterations": res.iterations, "converged": res.converged,
                      "true_rel_residual": res.true_residual_norm / bn,
                      "reliable_updates": res.reliable_updates,

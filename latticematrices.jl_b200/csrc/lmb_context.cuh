@@ -292,16 +292,28 @@ inline bool ensure_partials(lmb_ctx *ctx, size_t blocks, int nval) {
   return true;
 }
 
-// a field of V sites (default: the context's 4D volume)
+// a field of V sites in memory of field_bytes bytes (256-byte aligned)
 template <int P, int NC>
-inline bool make_field(lmb_ctx *ctx, const std::string &name, Field<P, NC> &f, int64_t V = -1, bool spare = false) {
+inline size_t field_bytes(int64_t V) {
+  const size_t n = Field<P, NC>::bytes(V) + Field<P, NC>::norm_bytes(V) + 256;
+  return (n + 255) / 256 * 256;
+}
+template <int P, int NC>
+inline Field<P, NC> field_at(void *mem, int64_t V) {
+  Field<P, NC> f;
+  f.V = V;
+  f.data = (decltype(f.data))mem;
+  f.norm = Field<P, NC>::norm_bytes(V) ? (float *)((char *)mem + (Field<P, NC>::bytes(V) + 255) / 256 * 256) : nullptr;
+  return f;
+}
+// and in a workspace (V: default the context's 4D volume)
+template <int P, int NC>
+inline bool make_field(lmb_ctx *ctx, const std::string &name, Field<P, NC> &f, int64_t V = -1) {
   if (V < 0) V = ctx->g.V;
   f.V = V;
-  const size_t nb = Field<P, NC>::bytes(V), mb = Field<P, NC>::norm_bytes(V);
-  void *p = (spare ? spare_workspace : workspace)(ctx, name, nb + mb + 256);
-  if (!p) return false;
-  f.data = (decltype(f.data))p;
-  f.norm = mb ? (float *)((char *)p + ((nb + 255) / 256) * 256) : nullptr;
+  void *mem = workspace(ctx, name, field_bytes<P, NC>(V));
+  if (!mem) return false;
+  f = field_at<P, NC>(mem, V);
   return true;
 }
 

@@ -11,9 +11,10 @@
 // above the pair) instead of two, and D5^+ exchanges half of Z through shared
 // memory instead of all of it.
 //
-// What bounds it: issue and latency, not DRAM (int16 D5 has 112 B per site to
-// move, 27 us at 16^3x32x12; its packed arithmetic alone takes about 85 us).
-// At that size a D5 takes 195 us on int16 fields (one site per thread: 242)
+// No unit stands at its limit: at 16^3x32x12 on int16 fields a D5 (a D5^+) issues
+// in 51 (49) % of the slots, the FMA pipe is 46 (45) % busy, L1 44 (36) %, and it
+// moves 0.8 (1.5) TB/s of DRAM and 6 (7) through L2, at 16 warps per SM; its
+// packed arithmetic alone takes about 85 us.  At that size a D5 takes 195 us on int16 fields (one site per thread: 242)
 // and a D5^+ with the CG update 178 (231); the solves take 217 ms on int16
 // (265) and 262 ms on FP32 fields (290).  The other way round, int16 on three
 // blocks of 168 registers and FP32 on four of 128, they take 223 and 284 ms;

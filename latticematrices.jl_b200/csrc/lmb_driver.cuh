@@ -29,6 +29,17 @@ int op_unpack_out(lmb_ctx *ctx, const Op &, void *dst, const Field<PS, NC> &f, c
 // the workspaces a precision's launches of the operator take inside a solve
 // (made before the solve spends memory it could do without)
 template <int PS, class Op> bool op_reserve(lmb_ctx *, const Op &) { return true; }
+// K2's epilogues of the operator's solves in storage PS: x in every iteration
+// (EpiCGUpdate), or for several iterations at once (EpiCGRing) where op_rings says
+// so, or always
+enum RingUse { RING_NEVER, RING_WHERE_IT_PAYS, RING_ALWAYS };
+template <class Op, int PS> struct UsesRing { static constexpr RingUse value = RING_NEVER; };
+template <int PS, class Op> bool op_rings(const lmb_ctx *, const Op &, int64_t /* bytes of a direction */) {
+  return false;
+}
+// Smaller directions stay in L2 with the rest, and their allocation takes as long
+// as a solve gains.
+constexpr int64_t kRingBytes = (int64_t)16 << 20;
 
 // all iterations up to the next status change in one launch (lmb_small.cuh):
 // LMB_OK or an error; kNotSmall, with nothing done, where the operator or the
@@ -334,31 +345,50 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
   int k1_n = 0, k2_n = 0;
 
   EpiStoreNorm<PS, NC> epi1{tl, ctx->st_dev, ctx->partials, ctx->counter};
-  // x += alpha p waits until `depth` of them have come together (EpiCGUpdate).
-  // The direction of an iteration with n of them waiting is ring[n].  The extra
+  // x += alpha p waits until `depth` of them have come together (EpiCGRing).  The
+  // direction of an iteration with n of them waiting is ring[n].  The extra
   // directions take at most 4 GiB of memory that nothing else of the solve asks
   // for; where there is none x is updated more often, and a later call that
   // runs out of memory takes them back (release_spare).
+  constexpr RingUse use = UsesRing<Op, PS>::value;
   Field<PS, NC> ring[kXDepth] = {p, p, p, p};
-  EpiCGUpdate<PS, PX, NC> epi2{{p, p, p, p}, rl, xl, ctx->st_dev, ctx->partials, ctx->counter};
+  EpiCGUpdate<PS, PX, NC> epi2{p, rl, xl, ctx->st_dev, ctx->partials, ctx->counter};
+  EpiCGRing<PS, PX, NC> epi2r{{p, p, p, p}, rl, xl, ctx->st_dev, ctx->partials, ctx->counter};
   int depth = 0;
   SpareHold hold(ctx);
   auto make_ring = [&]() -> bool {
-    static const char *const name[kXDepth] = {"cg_p", "cg_p1", "cg_p2", "cg_p3"};
     if (!op_reserve<PS>(ctx, op) || !op_reserve<PREC_DOUBLE>(ctx, op)) return false;
-    const int64_t want =
-        std::min(limit_of(ctx, "directions", kXDepth), 1 + ((int64_t)4 << 30) / (int64_t)Field<PS, NC>::bytes(V));
-    for (depth = 1; depth < want && make_field(ctx, name[depth], ring[depth], V, true); depth++)
-      epi2.p[depth] = ring[depth];
+    depth = 1;
+    if (use == RING_NEVER) return true;
+    const int64_t one = (int64_t)field_bytes<PS, NC>(V);
+    int64_t want = limit_of(ctx, "directions", INT64_MAX);
+    if (want == INT64_MAX && use == RING_WHERE_IT_PAYS && !op_rings<PS>(ctx, op, one)) want = 1;
+    want = std::min({want, (int64_t)kXDepth, 1 + ((int64_t)4 << 30) / one});
+    char *mem = nullptr;  // one allocation: each takes 0.3 ms of a first solve
+    while (want > 1 && !(mem = (char *)spare_workspace(ctx, "cg_ring", (want - 1) * one))) want--;
+    for (; depth < want; depth++) epi2r.p[depth] = ring[depth] = field_at<PS, NC>(mem + (depth - 1) * one, V);
     if (depth > 1) hold.take();
     return true;
   };
+  // K2 of an iteration after which every waiting update of x is made (all) or none
+  auto launch_k2 = [&](bool all) -> int {
+    if constexpr (use != RING_ALWAYS) {
+      if (depth == 1) return op.template launch<PS, 1>(ctx, tl, epi2, st);
+    }
+    if constexpr (use != RING_NEVER) {
+      epi2r.nx = all ? depth : 0;
+      return op.template launch<PS, 1>(ctx, tl, epi2r, st);
+    }
+    return LMB_OK;
+  };
   auto flush_x = [&]() -> int {
-    if (!hs->npend) return LMB_OK;
-    cg_x_update_kernel<PS, PX, NC><<<bgrid, kBlasThreads, 0, st>>>(epi2, ctx->st_dev, hs->npend, V);
-    LMB_CHECK_LAUNCH(ctx);
-    nl++;
-    LMB_CUDA(ctx, cudaMemsetAsync(&ctx->st_dev->npend, 0, sizeof(int), st));
+    if (use == RING_NEVER || !hs->npend) return LMB_OK;
+    if constexpr (use != RING_NEVER) {
+      cg_x_update_kernel<<<bgrid, kBlasThreads, 0, st>>>(epi2r, ctx->st_dev, hs->npend, V);
+      LMB_CHECK_LAUNCH(ctx);
+      nl++;
+      LMB_CUDA(ctx, cudaMemsetAsync(&ctx->st_dev->npend, 0, sizeof(int), st));
+    }
     return LMB_OK;
   };
   while (hs->status == ST_RUNNING) {
@@ -377,8 +407,7 @@ int cg_run(lmb_ctx *ctx, const lmb_cg_params *prm, const Op &op, void *x_pad, co
       if (rc) return rc;
       nl++;
       if (prm->profile) cudaEventRecord(pool.ev[4 * i + 1], st);
-      epi2.nx = last ? depth : 0;
-      rc = op.template launch<PS, 1>(ctx, tl, epi2, st);
+      rc = launch_k2(last);
       if (rc) return rc;
       nl++;
       if (prm->profile) cudaEventRecord(pool.ev[4 * i + 2], st);

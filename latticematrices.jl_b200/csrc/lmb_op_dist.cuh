@@ -16,6 +16,7 @@ template <class Epi> struct HasPairAdj { static constexpr bool value = false; };
 template <int PS> struct HasPairAdj<EpiStore<PS, 12>> { static constexpr bool value = true; };
 template <int PS> struct HasPairAdj<EpiStoreNorm<PS, 12>> { static constexpr bool value = true; };
 template <int PS, int PX> struct HasPairAdj<EpiCGUpdate<PS, PX, 12>> { static constexpr bool value = true; };
+template <int PS, int PX> struct HasPairAdj<EpiCGRing<PS, PX, 12>> { static constexpr bool value = true; };
 
 template <int P, int NC>
 int dist_exchange(lmb_ctx *ctx, const Field<P, NC> &in, const DistView &dv, GhostSpinors<P, NC> &gh,
@@ -331,6 +332,7 @@ struct DistStaggeredPolicy {
   bool links_finite(const lmb_ctx *ctx) const { return base.links_finite(ctx); }
 };
 
+template <int PS> struct UsesRing<DistWilsonPolicy, PS> { static constexpr RingUse value = RING_ALWAYS; };
 inline double *op_local_sums(const lmb_ctx *ctx, const DistWilsonPolicy &) { return ctx->dist->sums; }
 inline double *op_local_sums(const lmb_ctx *ctx, const DistStaggeredPolicy &) { return ctx->dist->sums; }
 inline int op_allreduce_sums(lmb_ctx *ctx, const DistWilsonPolicy &, cudaStream_t st) {

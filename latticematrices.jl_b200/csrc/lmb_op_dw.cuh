@@ -109,6 +109,12 @@ inline int64_t op_volume(const lmb_ctx *ctx, const DWPolicy &) { return ctx->g.V
 template <> struct DirectOut<DWPolicy> { static constexpr bool value = true; };
 inline int op_slices(const lmb_ctx *ctx, const DWPolicy &) { return ctx->dw_L5; }
 inline int64_t op_max_blocks(const lmb_ctx *ctx, const DWPolicy &) { return DWPolicy::max_blocks(ctx); }
+template <int PS> struct UsesRing<DWPolicy, PS> {
+  static constexpr RingUse value = PS == PREC_DOUBLE ? RING_NEVER : RING_WHERE_IT_PAYS;
+};
+template <int PS> bool op_rings(const lmb_ctx *ctx, const DWPolicy &, int64_t bytes) {
+  return bytes >= kRingBytes && DWPolicy::pairs<PS>(ctx);
+}
 template <int PS> bool op_reserve(lmb_ctx *ctx, const DWPolicy &) {
   Field<PS, 12> f;
   return DWPolicy::one_pass(ctx) || DWPolicy::make_tmp(ctx, f);

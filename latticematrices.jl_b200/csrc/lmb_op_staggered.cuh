@@ -13,6 +13,10 @@ template <> struct PairSiteAcc<EpiStoreOut<3>> { static constexpr bool value = t
 template <int NC> struct StagMinBlocks<double, EpiStoreOut<NC>> { static constexpr int value = 5; };  // as EpiStore
 template <> struct PairSiteAcc<EpiStoreNorm<PREC_DOUBLE, 3>> { static constexpr bool value = true; };
 template <> struct PairSiteAcc<EpiCGUpdate<PREC_DOUBLE, PREC_DOUBLE, 3>> { static constexpr bool value = true; };
+template <> struct PairSiteAcc<EpiCGRing<PREC_DOUBLE, PREC_DOUBLE, 3>> { static constexpr bool value = true; };
+template <int NC> struct StagMinBlocks<double, EpiCGRing<PREC_DOUBLE, PREC_DOUBLE, NC>> {
+  static constexpr int value = LMB_STAG_K2MINB;  // as EpiCGUpdate
+};
 
 struct StaggeredPolicy {
   static constexpr int NC = 3;
@@ -142,6 +146,11 @@ struct StaggeredPolicy {
 };
 
 template <> struct DirectOut<StaggeredPolicy> { static constexpr bool value = true; };
+// FP64, whose K2 is nearest to the bandwidth (figures at EpiCGRing)
+template <int PS> struct UsesRing<StaggeredPolicy, PS> {
+  static constexpr RingUse value = PS == PREC_DOUBLE ? RING_WHERE_IT_PAYS : RING_NEVER;
+};
+template <int PS> bool op_rings(const lmb_ctx *, const StaggeredPolicy &, int64_t bytes) { return bytes >= kRingBytes; }
 
 // small lattices (lmb_small_staggered.cu)
 template <int PS, int PX>

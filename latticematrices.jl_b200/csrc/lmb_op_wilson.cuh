@@ -99,6 +99,11 @@ struct WilsonPolicy {
 };
 
 template <> struct DirectOut<WilsonPolicy> { static constexpr bool value = true; };
+template <int PS> struct UsesRing<WilsonPolicy, PS> { static constexpr RingUse value = RING_WHERE_IT_PAYS; };
+// (figures at EpiCGRing; FP32 gains at every size that reaches the staged kernels)
+template <int PS> bool op_rings(const lmb_ctx *, const WilsonPolicy &, int64_t bytes) {
+  return PS == PREC_SINGLE || bytes >= kRingBytes;
+}
 // small lattices (lmb_small_wilson.cu)
 template <int PS, int PX>
 int op_cg_small(lmb_ctx *ctx, const WilsonPolicy &op, const Field<PS, 12> &p, const Field<PS, 12> &r,

@@ -209,20 +209,139 @@ struct EpiStoreNorm {  // K1
   }
 };
 
-// K2.  x enters no scalar of the iteration, so its updates are made for kXDepth
-// iterations at once, in their order (the same sum, rounding for rounding): x is
-// read and written a quarter as often, 288 of 2112 B per site and iteration of
-// the FP64 clover K2 and 144 of 640 B on int16 fields, and K3 writes the next
-// direction beside the ones that wait instead of over the last.  Bandwidth
-// bounds the FP64 K2, and it moves x's share no faster than the rest.  Solves,
-// updating x every 1, 2, 3, 4 iterations: clover FP64 24^3x48 226, 222, 219,
-// 218 ms, int16 32^3x64 283, 276, 274, 272, even/odd int16 24^3x48 34.6, 34.3,
-// 34.1, 34.1, HISQ FP32 32^3x64 185.6, 184.9, 184.2, 183.1, domain wall int16
-// 16^3x32x12 219, 216, 214, 214, Wilson FP64 16^3x32 15.0, 14.7, 14.5, 14.5.
-// (Loading x and p before r is stored, as an update in every iteration did,
-// spills 200 bytes here.)
 template <int PS, int PX, int NC = 12>
-struct EpiCGUpdate {
+struct EpiCGUpdate {  // K2
+  Field<PS, NC> p, r;
+  Field<PX, NC> x;
+  CGState *st;
+  double *partials;
+  unsigned *counter;
+  double *local = nullptr;  // as EpiStoreNorm::local
+  LMB_D bool skip() const { return ((volatile CGState *)st)->status != ST_RUNNING; }
+  LMB_D void finalize(double total) const { finalize_rr(st, total); }
+  template <typename R> LMB_D void operator()(int s, bool active, const Cx<R> *v) const {
+    double n2[1] = {0.0}, tot[1];
+    if (active) {
+      const R alpha = (R)st->alpha;
+      Cx<R> pv[NC], rv[NC], xv[NC];
+      p.load(s, pv);
+      r.load(s, rv);
+      x.load(s, xv);
+#pragma unroll
+      for (int k = 0; k < NC; k++) {
+        rv[k] = rv[k] - alpha * v[k];
+        xv[k] = xv[k] + alpha * pv[k];
+      }
+      r.store(s, rv);
+      x.store(s, xv);
+      n2[0] = sum_norm2(rv, NC);
+    }
+    if (grid_reduce<kDslashThreads, 1>(n2, partials, counter, tot) && threadIdx.x == 0) {
+      if (local) *local = tot[0];
+      else finalize_rr(st, tot[0]);
+    }
+  }
+  LMB_D void pair_adj(int s0, bool active, const Cx2 *v) const {
+    double n2[1] = {0.0};
+    pair_adj_acc(s0, active, v, n2);
+    finish(n2);
+  }
+  // one site: update and add |r|^2 to red (the FP64 pair stencils)
+  template <typename R> LMB_D void site_acc(int s, bool active, const Cx<R> *v, double (&red)[1]) const {
+    if (active) {
+      const R alpha = (R)st->alpha;
+      Cx<R> pv[NC], rv[NC], xv[NC];
+      p.load(s, pv);
+      r.load(s, rv);
+      x.load(s, xv);
+#pragma unroll
+      for (int k = 0; k < NC; k++) {
+        rv[k] = rv[k] - alpha * v[k];
+        xv[k] = xv[k] + alpha * pv[k];
+      }
+      r.store(s, rv);
+      x.store(s, xv);
+      red[0] += sum_norm2(rv, NC);
+    }
+  }
+  // persistent kernels: update and add |r|^2 to red; finish() once per block
+  LMB_D void pair_adj_acc(int s0, bool active, const Cx2 *v, double (&red)[1]) const {
+    if (active) {
+      const float a = (float)st->alpha;
+      const float2 pa = f2(a), na = f2(-a);
+      Cx2 pv[NC], rv[NC], xv[NC];
+      load_adj_rw(p, s0, pv);
+      load_adj_rw(r, s0, rv);
+      load_adj_rw(x, s0, xv);
+      float2 q = f2(0.f);
+#pragma unroll
+      for (int k = 0; k < NC; k++) {
+        rv[k] = Cx2(fma2(na, v[k].re, rv[k].re), fma2(na, v[k].im, rv[k].im));
+        xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
+        q = norm2_acc(rv[k], q);
+      }
+      store_adj(r, s0, rv);
+      store_adj(x, s0, xv);
+      red[0] += (double)q.x + (double)q.y;
+    }
+  }
+  LMB_D void finish(double (&red)[1]) const {
+    double tot[1];
+    if (grid_reduce<kDslashThreads, 1>(red, partials, counter, tot) && threadIdx.x == 0) {
+      if (local) *local = tot[0];
+      else finalize_rr(st, tot[0]);
+    }
+  }
+  LMB_D void pair(int s0, int s1, bool active, const Cx2 *v) const {
+    double n2[1] = {0.0}, tot[1];
+    if (active) {
+      const float a = (float)st->alpha;
+      const float2 pa = f2(a), na = f2(-a);
+      Cx2 pv[NC], rv[NC], xv[NC];
+      load2(p, s0, s1, pv);
+      load2(r, s0, s1, rv);
+      load2(x, s0, s1, xv);
+      float2 q = f2(0.f);
+#pragma unroll
+      for (int k = 0; k < NC; k++) {
+        rv[k] = Cx2(fma2(na, v[k].re, rv[k].re), fma2(na, v[k].im, rv[k].im));
+        xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
+        q = norm2_acc(rv[k], q);
+      }
+      store2(r, s0, s1, rv);
+      store2(x, s0, s1, xv);
+      n2[0] = (double)q.x + (double)q.y;
+    }
+    if (grid_reduce<kDslashThreads, 1>(n2, partials, counter, tot) && threadIdx.x == 0) {
+      if (local) *local = tot[0];
+      else finalize_rr(st, tot[0]);
+    }
+  }
+};
+
+// K2 with the updates of x of several iterations at once.  x enters no scalar of
+// the iteration, so x += alpha p can wait (npend, ahist in CGState) until up to
+// kXDepth of them are made in their order (the same sum, rounding for rounding):
+// x is read and written once for all, 288 of 2112 B per site and iteration of the
+// FP64 clover K2 and 144 of 640 B on int16 fields, and K3 writes the next
+// direction beside the ones that wait instead of over the last.  It pays where
+// K2's bytes do, and costs where K2 waits for its gathers: r is stored before x
+// and each p are loaded, one after another, where EpiCGUpdate loads all three at
+// once (which here spills 200 bytes).  So op_rings chooses.  Solves, x in every
+// iteration -> four directions, ms:
+//   Wilson FP64 16^3x32 15.2 -> 14.4, 24^4 35.0 -> 33.8; FP32 16^3x24 9.1 -> 8.7,
+//   24^4 25.2 -> 22.6; int16 16^3x32 9.25 -> 9.29, 24^3x32 21.4 -> 20.9; clover
+//   FP64 16^3x32 47.0 -> 43.9, FP32 24^4 68.4 -> 64.2, int16 16^3x32 21.8 -> 21.7,
+//   24^4 40.6 -> 39.8, 24^3x32 53.6 -> 52.3; even/odd clover FP64 18^2x20^2 17.8 ->
+//   17.5, 24^3x48 77.8 -> 76.5, int16 pairs 24^3x48 34.5 -> 34.2; domain wall pairs
+//   16^4x12 int16 84.5 -> 83.8, FP32 101.2 -> 100.3; HISQ FP64 24^3x32 43.0 -> 42.2,
+//   32^4 108.2 -> 105.4.
+//   Taken nowhere: staggered FP32 24^3x32 19.7 -> 20.1, int16 18.3 -> 19.0, HISQ
+//   int16 21.2 -> 21.6, domain wall one site int16 12^3x16x9 35.3 -> 35.9, even/odd
+//   FP32 12^2x16^2 6.1 -> 6.4.
+// (The sharded operators have only this epilogue, with four directions always.)
+template <int PS, int PX, int NC>
+struct EpiCGRing {
   Field<PS, NC> p[kXDepth], r;
   Field<PX, NC> x;
   CGState *st;
@@ -251,6 +370,19 @@ struct EpiCGUpdate {
         for (int k = 0; k < NC; k++) xv[k] = xv[k] + a * pv[k];
       }
     x.store(s, xv);
+  }
+  LMB_D void add_x2(int s0, int s1) const {
+    Cx2 xv[NC], pv[NC];
+    load2(x, s0, s1, xv);
+#pragma unroll
+    for (int j = 0; j < kXDepth; j++)
+      if (j < nx) {
+        const float2 pa = f2((float)alpha_of(j));
+        load2(p[j], s0, s1, pv);
+#pragma unroll
+        for (int k = 0; k < NC; k++) xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
+      }
+    store2(x, s0, s1, xv);
   }
   LMB_D void add_x_adj(int s0) const {
     Cx2 xv[NC], pv[NC];
@@ -284,7 +416,7 @@ struct EpiCGUpdate {
 #pragma unroll
       for (int k = 0; k < NC; k++) rv[k] = rv[k] - alpha * v[k];
       r.store(s, rv);
-      red[0] += sum_norm2(rv, NC);
+      red[0] += sum_norm2(rv, NC);  // before x: r's registers are free then
       if (nx) add_x<R>(s);
     }
   }
@@ -326,19 +458,7 @@ struct EpiCGUpdate {
       }
       store2(r, s0, s1, rv);
       n2[0] = (double)q.x + (double)q.y;
-      if (nx) {
-        Cx2 xv[NC], pv[NC];
-        load2(x, s0, s1, xv);
-#pragma unroll
-        for (int j = 0; j < kXDepth; j++)
-          if (j < nx) {
-            const float2 pa = f2((float)alpha_of(j));
-            load2(p[j], s0, s1, pv);
-#pragma unroll
-            for (int k = 0; k < NC; k++) xv[k] = Cx2(fma2(pa, pv[k].re, xv[k].re), fma2(pa, pv[k].im, xv[k].im));
-          }
-        store2(x, s0, s1, xv);
-      }
+      if (nx) add_x2(s0, s1);
     }
     finish(n2);
   }
@@ -430,6 +550,7 @@ struct EpiTrueResidual {
 template <class Epi> struct ReducingEpi { static constexpr bool value = false; };
 template <int PS, int NC> struct ReducingEpi<EpiStoreNorm<PS, NC>> { static constexpr bool value = true; };
 template <int PS, int PX, int NC> struct ReducingEpi<EpiCGUpdate<PS, PX, NC>> { static constexpr bool value = true; };
+template <int PS, int PX, int NC> struct ReducingEpi<EpiCGRing<PS, PX, NC>> { static constexpr bool value = true; };
 template <int NC> struct ReducingEpi<EpiResidualNorm<NC>> { static constexpr bool value = true; };
 template <int PS, int NC> struct ReducingEpi<EpiTrueResidual<PS, NC>> { static constexpr bool value = true; };
 
@@ -489,12 +610,11 @@ __global__ void __launch_bounds__(kBlasThreads)
   dst.store(s, b);
 }
 
-// x64 += x_low; x_low = 0
 // the iterations whose x += alpha p is still to be added (a solve that pauses
 // or ends between two updates of x)
 template <int PS, int PX, int NC>
 __global__ void __launch_bounds__(kBlasThreads)
-    cg_x_update_kernel(const EpiCGUpdate<PS, PX, NC> epi, const CGState *st, int n, int64_t V) {
+    cg_x_update_kernel(const EpiCGRing<PS, PX, NC> epi, const CGState *st, int n, int64_t V) {
   const int64_t s = (int64_t)blockIdx.x * kBlasThreads + threadIdx.x;
   if (s >= V) return;
   typedef typename Real<PS>::type R;
@@ -509,6 +629,7 @@ __global__ void __launch_bounds__(kBlasThreads)
   epi.x.store(s, xv);
 }
 
+// x64 += x_low; x_low = 0
 template <int PX, int NC>
 __global__ void __launch_bounds__(kBlasThreads)
     fold_kernel(Field<PREC_DOUBLE, NC> x, Field<PX, NC> xl, int64_t V) {

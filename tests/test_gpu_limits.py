@@ -106,10 +106,12 @@ def _fits(lmb, call):
 # Every number of directions, and every number of updates of x that still wait
 # when the solve pauses or stops: the same sum in the same order.  A solve that
 # stops with some of them waiting launches one kernel more, which shows how many
-# directions it ran with.
-@pytest.mark.parametrize("solve", [_clover_solve, _staggered_solve])
+# directions it ran with (storages whose solves take no extra ones: one).
+@pytest.mark.parametrize("solve,storages", [(_clover_solve, ("double", "single", "half")),
+                                            (_evenodd_solve, ("double", "half")),
+                                            (_domainwall_solve, ("single", "half")), (_staggered_solve, ("double",))])
 @pytest.mark.parametrize("precision", ["double", "single", "half"])
-def test_solution_does_not_depend_on_the_directions(lmb, orc, monkeypatch, solve, precision):
+def test_solution_does_not_depend_on_the_directions(lmb, orc, monkeypatch, solve, storages, precision):
     monkeypatch.setenv("LMB_PERSISTENT", "0")
     for maxiter in (2, 3, 4, 300):
         out = []
@@ -120,9 +122,32 @@ def test_solution_does_not_depend_on_the_directions(lmb, orc, monkeypatch, solve
         for res, (x,) in out[1:]:
             assert (res.iterations, res.reason) == (out[0][0].iterations, out[0][0].reason)
             np.testing.assert_array_equal(x, out[0][1][0])
-        if precision == "double" and maxiter < 300:
+        if maxiter < 300 and out[0][0].reliable_updates == 0:
             more = [res.kernel_launches - out[0][0].kernel_launches for res, _ in out]
-            assert more == [1 if maxiter % n else 0 for n in (1, 2, 3, 4)]
+            assert more == [1 if precision in storages and maxiter % n else 0 for n in (1, 2, 3, 4)]
+
+
+# Which solves take the extra directions, by the device memory that is gone
+# after them: three more fields of 16 V NC bytes (FP64) from 16 MiB a field on,
+# none below, as many as LMB_LIMITS says where it does.
+@pytest.mark.parametrize("L,limits,extra", [((16, 16, 16, 16), "", 0), ((16, 16, 16, 24), "", 3),
+                                            ((16, 16, 16, 16), "directions=4", 3), ((16, 16, 16, 24), "directions=2", 1)])
+def test_who_takes_extra_directions(lmb, monkeypatch, L, limits, extra):
+    import torch
+    U, b = lmb.random_su3_links(L, 0.25, 23), lmb.gaussian_fermion(L, 3, 4, 24, phases=PHASES)
+    x, t = b.similar(), b.similar()
+
+    def taken(limits):
+        monkeypatch.setenv("LMB_LIMITS", limits)
+        D = lmb.WilsonDiracOperator4D(U, 0.12)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        lmb.cg_(x, lmb.DdagDOp(D, t), b, maxiter=2)
+        return before - torch.cuda.mem_get_info()[0]
+    monkeypatch.setenv("LMB_PERSISTENT", "0")
+    taken("directions=1")  # what the process allocates once
+    got = taken(limits) - taken("directions=1")
+    assert abs(got - extra * 192 * np.prod(L)) <= 1 << 22  # device pages of 2 MiB
 
 
 # The extra directions are no reason for a call to run out of memory: neither
