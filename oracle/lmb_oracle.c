@@ -771,9 +771,9 @@ void orc_cg_ddagd(const orc_operator *op, double *x, const double *b,
   double bn = sqrt(bb);
   double tol = fmax(atol, rtol * bn);
   orc_apply_ddagd(op, x, tmp, Ap);
-  axpby_real(n, 1.0, b, 0.0, r);
+  memcpy(r, b, sizeof(double) * n); /* 0 times fresh memory may be NaN */
   axpby_real(n, -1.0, Ap, 1.0, r);
-  axpby_real(n, 1.0, r, 0.0, p);
+  memcpy(p, r, sizeof(double) * n);
   double rr = re_dot(n, r, r);
   if (!isfinite(rr) || rr < 0) {
     cg_finish(res, 0, 0, NAN, bn, 3);

@@ -285,6 +285,17 @@ def test_cg_ddagd_true_residual(orc):
     assert resz["relative_residual"] == 0.0
 
 
+def test_cg_ddagd_does_not_read_fresh_memory(orc):
+    """Its work vectors come from memory that held NaN before."""
+    L = (4, 4, 4, 4)
+    U, b = orc.random_su3_links(L, 0.3, 1), orc.gaussian_field(L, 3, 4, 2)
+    op = orc.Operator(orc.OP_WILSON, U, L, kappa=0.125)
+    for _ in range(3):
+        junk = [np.full(b.size, np.nan + 1j * np.nan) for _ in range(16)]
+        del junk
+        assert orc.cg_ddagd(op, b)[1]["converged"]
+
+
 def test_random_links_are_su3_and_seeded(orc):
     L = (2, 2, 2, 2)
     U = orc.random_su3_links(L, 0.2, 1)
